@@ -8,238 +8,290 @@
 // on the GPU:
 //
 //   * The factor is cut into 64 x 64 tiles (the last row and column ragged).
-//     A task produces one finished tile L_ij (i >= j):
-//         S    = A_ij - sum_{k<j} L_ik L_jk^T          (SYRK for i == j, GEMMs otherwise)
-//         i==j : L_jj = potrf(S), W_j = L_jj^-1       (POTRF, and the inverse for the tiles below)
-//         i> j : L_ij = S W_j^T                       (TRSM as a product with the inverse)
-//     The sum runs left-looking in 32-column chunks on DMMA (mma.sync
-//     m16n8k4 f64), each chunk staged by cp.async once the two tiles it reads
-//     are final.
-//   * Tasks are handed out by an atomic ticket in column order, the diagonal
-//     task first in each column: the device form of the reference's priorities
-//     (the critical POTRF/TRSM chain of column j goes out before any work of
-//     column j+1).  A task waits only on tiles of earlier columns and on the
-//     diagonal tile of its own column, all with smaller tickets, which running
-//     CTAs hold; so the walk cannot deadlock whatever the residency.
-//   * Every tile has a done flag (release by one thread after a CTA barrier,
-//     acquire by one thread before a CTA barrier).  Every wait is bounded by
-//     wait_ns of device time; a wait that runs out sets st->timeout and the
-//     CTA drains its copies and stops, and the other waiters see the timeout
-//     and stop too.
+//     Two kinds of tasks, both left-looking:
+//       T(i, j), i >= j + 2:  S = A_ij - sum_{k<j} L_ik L_jk^T,  L_ij = S W_j^T
+//       M(j):  L_{j,j-1} the same way, then
+//              S = A_jj - sum_{k<j} L_jk L_jk^T,  L_jj = potrf(S),  W_j = L_jj^-1
+//     M(j) holds the whole critical path of column j: both tiles accumulate
+//     side by side while column j-1 is being factored, and once W_{j-1} is
+//     there the sub-diagonal tile goes from the TRSM product through shared
+//     memory into the diagonal tile's update and its factor, without a trip
+//     through global memory and a flag in between.
+//   * The sums run in 16-column chunks on DMMA (mma.sync m16n8k4 f64) through a
+//     4-stage cp.async ring, each chunk issued once the two tiles it reads are
+//     final.
+//   * Tasks are handed out by an atomic ticket: M(0), M(1), then per column c
+//     T(c+2, c), M(c+2), T(c+3, c), ...: the device form of the reference's
+//     priorities (the POTRF/TRSM chain goes out two columns ahead of the rest).
+//     A task waits only on tiles with smaller tickets, which running CTAs hold;
+//     so the walk cannot deadlock whatever the residency.
+//   * The tiles of a row are finished in column order (tile (i, k) needs every
+//     (i, k' < k)), so one counter per row says how many are final.  It is set
+//     by a release of one thread after a CTA barrier and read by an acquire of
+//     one thread before one; a CTA keeps the value it saw and polls again only
+//     past it.  Every wait is bounded by wait_ns of device time; a wait that
+//     runs out sets st->timeout and the CTA drains its copies and stops, and the
+//     other waiters see the timeout and stop too.
 //   * A non-positive pivot is reported LAPACK-style in st->info (1-based
 //     global column); the columns before it are final for every row, and the
-//     walk still finishes every task (with the inverse's rows past the failure
-//     replaced by identity rows), so nothing waits forever.
+//     walk still finishes every task (with the inverse's rows from the failure
+//     on replaced by identity rows), so nothing waits forever.
 #include "common.cuh"
 
 namespace lnb {
 namespace dag {
 
 constexpr int TS = 64;              // tile order
-constexpr int NT = 128;             // threads per CTA (4 warps, 2 x 2 warp grid of 32 x 32)
-constexpr int BK = 32;              // K chunk
+constexpr int NT = 128;             // threads per CTA (4 warps)
+constexpr int BK = 16;              // K chunk
+constexpr int ST = 4;               // stages of the chunk ring
 constexpr int LDK = TS + 4;         // k-major staged rows (= 4 mod 16 doubles: conflict-free fragments)
 constexpr int CHUNK = BK * LDK;     // doubles per staged operand chunk
-constexpr int LDS = TS + 1;         // row-major tile for the diagonal factor
-constexpr int SMEM_STAGES = 2 * 2 * CHUNK * (int)sizeof(double);          // 2 stages x {A, B}
-constexpr int SMEM_POTRF = (2 * TS * LDS + 32) * (int)sizeof(double);     // S, W and the pivot reciprocals
-constexpr int SMEM = SMEM_STAGES > SMEM_POTRF ? SMEM_STAGES : SMEM_POTRF;
+constexpr int HALF = TS * LDK;      // a whole 64 x 64 tile, k-major
+constexpr int PW = 8;               // panel width of the diagonal factor
+constexpr uint64_t YIELD_NS = 40000;
+constexpr int NBUSY = 256;          // SMs told apart by the busy flags
+constexpr int LDX = 10;             // column stride of a panel's 8 x 8 inverse
+static_assert(2 * HALF == 2 * ST * CHUNK, "the epilogue's two tiles fill the ring");
+constexpr int SMEM = (2 * HALF + 2 * PW * LDX) * (int)sizeof(double);
 
 struct Args {
     double *A;
     int64_t lda, n;
     int nt, ntasks;
     double *W;              // nt inverses of the diagonal tiles, 64 x 64 column-major each
-    int *done;              // done[k * nt + i]: tile (i, k) is final
+    int *prog;              // prog[i]: tiles (i, 0 .. prog[i]-1) are final
+    int *busy;              // busy[sm]: a task on that SM is in its critical section
     int *ticket;
     int ticket0;            // first ticket handed out (0; 1 only in the wait self-test)
     lnb_status_t *st;
     long long wait_ns;
 };
 
-// ---- one warp: Cholesky of a 32 x 32 block and its inverse ------------------
-// S: row-major (ld lds), lower part read and written.  X: row-major (ld ldx),
-// receives inv(L) (lower; zeros above).  rd: 32 doubles of scratch.
-// Factor: lane r owns row r in registers; a runtime loop over the columns
-// keeps a[0] the current column (the array shifts down by one per step, so
-// every index is a compile-time constant) and reads L's finished column back
-// from shared memory, where every lane reads the same word (a broadcast).
-// Inverse: lane q forms column q of inv(L) by forward substitution with the
-// stored reciprocal pivots, X[r][q] = (delta_rq - sum_{k<r} L[r][k] X[k][q]) / L[r][r].
-// Returns the local column of the first non-positive pivot, or 32.  After a
-// failure the failed pivot and the columns after it keep their updated values
-// (LAPACK's potf2 stops there) and X's rows from the failure on are identity
-// rows.
-LNB_DEV int warp_potrf32_inv(double *S, int lds, double *X, int ldx, double *rd)
+struct Shared {
+    int task, fail;
+    int known[2];
+};
+
+// 1/sqrt(d) for a normal d > 0: the approximate instruction (relative error
+// 2^-20 measured) and one third-order step of the iteration
+// y' = y (1 + h/2 + 3 h^2/8), h = 1 - d y^2 (Householder's method for y^-2 = d),
+// which leaves the last rounding (1.4e-16 measured).  No branch: rsqrt()'s
+// special-case branch would fence the column's other work off its latency.
+LNB_DEV double pivot_rsqrt(double d)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double h = fma(-(d * y), y, 1.0);
+    return fma(fma(0.375, h, 0.5), y * h, y);
+}
+
+// Columns 8p .. 8p+7 of the 64 x 64 tile Sc (column-major, ld LDK) for every
+// row from 8p down, and the inverse of their 8 x 8 diagonal block: X =
+// inv(L_pp)^T, Xs[c * LDX + r], comes out of the same column steps applied to
+// eight identity rows.  A warp holds the eight pivot rows in lanes 0-7 and 48 of
+// the other rows (the identity rows first) in the other lanes, two per lane;
+// panels 0 and 1 take two warps, which repeat the pivot rows and so need not
+// wait for each other.  Every lane tracks the pivots (dd): it takes the pivot
+// rows' entries of the column by shuffle before they are scaled, so the chain
+// per column is 1/sqrt -> multiply -> fma, and the shuffles and the rows'
+// updates run beside it.  The fast form takes every pivot as a normal positive
+// number and looks at them after the last column (a branch or a select per
+// column costs 100 - 270 of its 760 cycles); where one is not, it stores
+// nothing and the other form repeats the panel.  Returns the tile column of the
+// first non-positive pivot (its column and those after it keep their values),
+// 64 if there is none, or -1 (fast form) to ask for the repetition.
+LNB_DEV int panel_warps(int p) { return p < 2 ? 2 : 1; }
+template <bool FAST>
+LNB_DEV int warp_panel8(double *Sc, double *Xs, int p, int w)
 {
     const int lane = threadIdx.x & 31;
-    double a[32];
+    const int i0 = lane - PW + 48 * w, i1 = i0 + 24;         // identity rows 0-7, then rows 8p + 8 ..
+    const int row0 = PW * p + (lane < PW ? lane : i0), row1 = PW * p + i1;
+    const bool ident = lane >= PW && i0 < PW, real0 = !ident && row0 < TS, real1 = lane >= PW && row1 < TS;
+    double *col0 = Sc + PW * p * LDK + (real0 ? row0 : 0), *col1 = Sc + PW * p * LDK + (real1 ? row1 : 0);
+    double a[PW], b[PW], dd[PW];
 #pragma unroll
-    for (int k = 0; k < 32; ++k) a[k] = (k <= lane) ? S[lane * lds + k] : 0.0;
-    int fail = 32;
+    for (int k = 0; k < PW; ++k) {
+        a[k] = col0[k * LDK];
+        b[k] = col1[k * LDK];
+        if (!real0) a[k] = ident && k == i0 ? 1.0 : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < PW; ++k) dd[k] = __shfl_sync(0xffffffffu, a[k], k);
+    int fail = TS;
+#pragma unroll
+    for (int c = 0; c < PW; ++c) {
+        double s[PW];
+#pragma unroll
+        for (int k = c + 1; k < PW; ++k) s[k] = __shfl_sync(0xffffffffu, a[c], k);
+        double rs, rt;
+        if (FAST) {
+            rs = rt = pivot_rsqrt(dd[c]);
+        } else {
+            if (!(dd[c] > 0.0) && fail == TS) fail = PW * p + c;
+            rt = fail == TS ? rsqrt(dd[c]) : 0.0;            // a failed column updates nothing
+            rs = fail == TS ? rt : 1.0;
+        }
+        a[c] *= rs;
+        b[c] *= rs;
+#pragma unroll
+        for (int k = c + 1; k < PW; ++k) {
+            s[k] *= rt;
+            dd[k] = fma(-s[k], s[k], dd[k]);
+            a[k] = fma(-a[c], s[k], a[k]);
+            b[k] = fma(-b[c], s[k], b[k]);
+        }
+    }
+    if (FAST) {
+        double lo = dd[0];                                   // a NaN fails the comparison below
+#pragma unroll
+        for (int c = 1; c < PW; ++c) lo = dd[c] < lo || !(dd[c] == dd[c]) ? dd[c] : lo;
+        if (!(lo >= 2.2250738585072014e-308)) return -1;     // warp-uniform: dd is broadcast
+    }
+    if (ident) {
+#pragma unroll
+        for (int c = 0; c < PW; ++c) Xs[c * LDX + i0] = a[c];
+    } else if (real0 && (w == 0 || lane >= PW)) {
+#pragma unroll
+        for (int c = 0; c < PW; ++c)
+            if (lane >= c) col0[c * LDK] = a[c];
+    }
+    if (real1) {
+#pragma unroll
+        for (int c = 0; c < PW; ++c) col1[c * LDK] = b[c];
+    }
+    return fail;
+}
+__device__ __noinline__ int warp_panel8_checked(double *Sc, double *Xs, int p, int w)
+{
+    return warp_panel8<false>(Sc, Xs, p, w);
+}
+
+// acc, acc2 += A^T B over the staged rows [k0, k1) (k1 - k0 a multiple of 8): a
+// at column m, b at column n of two k-major tiles, eight rows of operands in
+// flight and two accumulators against the DMMA latency
+LNB_DEV void dot_tile(double (&acc)[4], double (&acc2)[4], const double *Am, const double *Bn, int k0, int k1, int t)
+{
+    if (k0 >= k1) return;
+    const double *ap = Am + (k0 + t) * LDK, *bp = Bn + (k0 + t) * LDK;
+    double x0 = ap[0], x1 = ap[8], xb = bp[0], y0 = ap[4 * LDK], y1 = ap[4 * LDK + 8], yb = bp[4 * LDK];
 #pragma unroll 1
-    for (int c = 0; c < 32; ++c) {
-        const double d = __shfl_sync(0xffffffffu, a[0], c);
-        if (!(d > 0.0)) {                                // warp-uniform: stop here
-            fail = c;
-#pragma unroll
-            for (int k = 0; k < 32; ++k)
-                if (c + k <= lane) S[lane * lds + c + k] = a[k];
-            break;
-        }
-        const double rs = rsqrt(d);
-        if (lane >= c) S[lane * lds + c] = (lane == c) ? d * rs : a[0] * rs;
-        if (lane == c) rd[c] = rs;
-        const double l = a[0] * rs;
+    for (int k = k0 + 8; k < k1; k += 8) {
+        ap += 8 * LDK;
+        bp += 8 * LDK;
+        const double u0 = ap[0], u1 = ap[8], ub = bp[0], v0 = ap[4 * LDK], v1 = ap[4 * LDK + 8], vb = bp[4 * LDK];
+        dmma16x8x4(acc, x0, x1, xb);
+        dmma16x8x4(acc2, y0, y1, yb);
+        x0 = u0; x1 = u1; xb = ub; y0 = v0; y1 = v1; yb = vb;
+    }
+    dmma16x8x4(acc, x0, x1, xb);
+    dmma16x8x4(acc2, y0, y1, yb);
+}
+
+// The CTA: factor the 64 x 64 tile Sc (column-major, ld LDK, lower part) in
+// place and store its inverse to Wg (column-major, global).  Bound by latency:
+// 64 dependent pivots.  In period p, panel_warps(p) warps factor panel p; the
+// others subtract the columns before it from panel p+1 (left-looking, one m16
+// row tile per job) and form E - L_p,<p W, rows 8p..8p+7 of the inverse up to the
+// factor inv(L_pp), as a transpose so that the tensor cores' N = 8 is the panel
+// and M the columns of W (one 16-column tile per job).  Only the last 8 columns'
+// two DMMA steps, the product with inv(L_pp) beside them and two barriers sit
+// between two panels.  Wr: 64 x LDK
+// doubles of scratch (rows of W); the caller zeroes W above its diagonal
+// 16 x 16 blocks.  panels: 8, or fewer to run the code on a dummy tile.  Returns the first failed column, or 64.
+LNB_DEV int cta_factor64(double *Sc, double *Wr, double *Xs2, double *Wg, int *s_fail, int panels)
+{
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+    auto finish_w = [&](int p, int qt) {             // W rows of panel p, columns of tile qt
+        const int q = 16 * qt + g, r = PW * p + 2 * t;
+        const double *Xs = Xs2 + (p & 1) * PW * LDX + g * LDX + t, *a = Wr + (PW * p + t) * LDK + q;
+        double o[4] = {0.0, 0.0, 0.0, 0.0};
+        const double a0 = a[0], a1 = a[8], a2 = a[4 * LDK], a3 = a[4 * LDK + 8], x0 = Xs[0], x1 = Xs[4];
+        dmma16x8x4(o, a0, a1, x0);
+        dmma16x8x4(o, a2, a3, x1);
         __syncwarp();
-#pragma unroll
-        for (int k = 1; k < 32; ++k) {
-            const double lk = S[((c + k) & 31) * lds + c];
-            if (c + k <= lane) a[k] = fma(-l, lk, a[k]);
+        double *wo = Wr + r * LDK + q, *go = Wg + r + TS * q;
+        wo[0] = o[0];
+        wo[LDK] = o[1];
+        wo[8] = o[2];
+        wo[LDK + 8] = o[3];
+        *reinterpret_cast<double2 *>(go) = make_double2(o[0], o[1]);
+        *reinterpret_cast<double2 *>(go + 8 * TS) = make_double2(o[2], o[3]);
+    };
+    if (tid == 0) *s_fail = TS;
+    int p = 0, fail = TS;
+#pragma unroll 1
+    for (;; ++p) {
+        const int np = panel_warps(p);
+        const int pn = p + 1, m0 = pn / 2, nupd = (p > 0 && pn < panels) ? 4 - m0 : 0;
+        if (w < np) {
+            int f = warp_panel8<true>(Sc, Xs2 + (p & 1) * PW * LDX, p, w);
+            if (f < 0) f = warp_panel8_checked(Sc, Xs2 + (p & 1) * PW * LDX, p, w);
+            if (f < TS && tid == 0) *s_fail = f;
+        } else {
+            // the longest sums first: W's tile 0, then S, then W's other tiles;
+            // a second round goes in reverse order
+            const int njobs = nupd + p / 2 + 1, ns = 4 - np;
+#pragma unroll 1
+            for (int rnd = 0; rnd * ns < njobs; ++rnd) {
+                const int job = rnd * ns + ((rnd & 1) ? NT / 32 - 1 - w : w - np);
+                if (job >= njobs) continue;
+                const bool upd = job > 0 && job <= nupd;
+                const int qt = job > 0 ? job - nupd : 0;
+                const int m = 16 * (upd ? m0 + job - 1 : qt) + g, pc = PW * (upd ? pn : p), c = pc + 2 * t;
+                double *T = (upd ? Sc : Wr) + m;
+                double *o0 = T + c * LDK, *o1 = o0 + LDK;
+                double acc[4] = {0.0, 0.0, 0.0, 0.0}, acc2[4] = {0.0, 0.0, 0.0, 0.0};
+                double e0 = m == c ? 1.0 : 0.0, e1 = m == c + 1 ? 1.0 : 0.0, e2 = m + 8 == c ? 1.0 : 0.0,
+                       e3 = m + 8 == c + 1 ? 1.0 : 0.0;
+                if (upd) {
+                    e0 = o0[0]; e1 = o1[0]; e2 = o0[8]; e3 = o1[8];
+                }
+                // W is zero above its diagonal
+                dot_tile(acc, acc2, T, Sc + pc + g, upd ? 0 : 16 * qt, PW * p, t);
+                o0[0] = e0 - (acc[0] + acc2[0]);
+                o1[0] = e1 - (acc[1] + acc2[1]);
+                o0[8] = e2 - (acc[2] + acc2[2]);
+                o1[8] = e3 - (acc[3] + acc2[3]);
+            }
         }
-#pragma unroll
-        for (int k = 0; k < 31; ++k) a[k] = a[k + 1];
-        a[31] = 0.0;
+        __syncthreads();                             // panel p is final
+        fail = *s_fail;
+        if (pn == panels || fail < TS) break;
+        if (w >= m0) {                               // panel p's own columns
+            const int m = 16 * w + g;
+            const double *a = Sc + (PW * p + t) * LDK;
+            double *o0 = Sc + (PW * pn + 2 * t) * LDK + m, *o1 = o0 + LDK;
+            double acc[4] = {0.0, 0.0, 0.0, 0.0}, acc2[4] = {0.0, 0.0, 0.0, 0.0};
+            dmma16x8x4(acc, a[m], a[m + 8], a[PW * pn + g]);
+            dmma16x8x4(acc2, a[4 * LDK + m], a[4 * LDK + m + 8], a[4 * LDK + PW * pn + g]);
+            o0[0] -= acc[0] + acc2[0];
+            o1[0] -= acc[1] + acc2[1];
+            o0[8] -= acc[2] + acc2[2];
+            o1[8] -= acc[3] + acc2[3];
+        }
+        if (w <= p / 2) finish_w(p, w);
+        __syncthreads();
     }
-    __syncwarp();
-    double x[32];
-#pragma unroll
-    for (int r = 0; r < 32; ++r) {
-        double sum = (r == lane) ? 1.0 : 0.0;
-#pragma unroll
-        for (int k = 0; k < r; ++k) sum = fma(-S[r * lds + k], x[k], sum);
-        x[r] = (r < fail) ? sum * rd[r < fail ? r : 0] : ((r == lane) ? 1.0 : 0.0);
+    if (w <= p / 2) finish_w(p, w);
+    if (fail < TS) {                                 // identity rows from the failure on
+        __syncthreads();
+        for (int idx = tid; idx < TS * TS; idx += NT)
+            if ((idx & 63) >= fail) Wg[idx] = (idx & 63) == (idx >> 6) ? 1.0 : 0.0;
     }
-#pragma unroll
-    for (int r = 0; r < 32; ++r) X[r * ldx + lane] = (r >= lane) ? x[r] : 0.0;
-    __syncwarp();
     return fail;
 }
 
-// ---- the CTA: factor and invert the 64 x 64 tile S (row-major, ld LDS) -------
-// 2 x 2 blocks of 32:  L00 = potrf(S00);  L10 = S10 W00^T;  S11 -= L10 L10^T;
-// L11 = potrf(S11);  W10 = -W11 (L10 W00).  W (row-major, ld LDS) receives
-// inv(L).  Returns the first failed local column, or 64.
-LNB_DEV int cta_potrf64_inv(double *S, double *W, int *s_fail, double *rd)
-{
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int idx = tid; idx < 32 * 32; idx += NT) W[(idx >> 5) * LDS + 32 + (idx & 31)] = 0.0;
-    if (warp == 0) {
-        const int f = warp_potrf32_inv(S, LDS, W, LDS, rd);
-        if (lane == 0) s_fail[0] = f;
-    }
-    __syncthreads();
-    const int f0 = s_fail[0];
-    // L10[r][c] = sum_{p <= c} S10[r][p] W00[c][p]; thread: row 32 + lane, columns 8 warp .. + 8
-    {
-        const int r = 32 + lane, cb = 8 * warp;
-        double o[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) o[u] = 0.0;
-        for (int p = 0; p < 32; ++p) {
-            const double s = S[r * LDS + p];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) o[u] = fma(s, W[(cb + u) * LDS + p], o[u]);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 8; ++u) S[r * LDS + cb + u] = o[u];
-    }
-    __syncthreads();
-    if (f0 < 32) {
-        // the trailing block is not factored: W11 = I, W10 = 0
-        for (int idx = tid; idx < 32 * 64; idx += NT) {
-            const int r = 32 + idx / 64, q = idx % 64;
-            W[r * LDS + q] = (q == r) ? 1.0 : 0.0;
-        }
-        __syncthreads();
-        return f0;
-    }
-    // S11 -= L10 L10^T on the lower part; thread: row 32 + lane, columns 32 + 8 warp .. + 8
-    {
-        const int r = 32 + lane, cb = 32 + 8 * warp;
-        double o[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) o[u] = 0.0;
-        for (int p = 0; p < 32; ++p) {
-            const double s = S[r * LDS + p];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) o[u] = fma(s, S[(cb + u) * LDS + p], o[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (r >= cb + u) S[r * LDS + cb + u] -= o[u];
-    }
-    __syncthreads();
-    if (warp == 0) {
-        const int f = warp_potrf32_inv(S + 32 * LDS + 32, LDS, W + 32 * LDS + 32, LDS, rd);
-        if (lane == 0) s_fail[1] = f;
-    }
-    __syncthreads();
-    const int f1 = s_fail[1];
-    // T = L10 W00 into the unused upper-right block of S: T[r][q] = sum_{p >= q} L10[r][p] W00[p][q]
-    {
-        const int r = lane, qb = 8 * warp;
-        double o[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) o[u] = 0.0;
-        for (int p = 0; p < 32; ++p) {
-            const double l = S[(32 + r) * LDS + p];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) o[u] = fma(l, W[p * LDS + qb + u], o[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) S[r * LDS + 32 + qb + u] = o[u];
-    }
-    __syncthreads();
-    // W10[r][q] = -sum_{s <= r} W11[r][s] T[s][q]
-    {
-        const int r = lane, qb = 8 * warp;
-        double o[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) o[u] = 0.0;
-        for (int s = 0; s < 32; ++s) {
-            const double w = W[(32 + r) * LDS + 32 + s];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) o[u] = fma(w, S[s * LDS + 32 + qb + u], o[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) W[(32 + r) * LDS + qb + u] = -o[u];
-    }
-    __syncthreads();
-    return f1 < 32 ? 32 + f1 : 64;
-}
-
-// ---- DMMA over one staged chunk: acc(64 x 64) += As^T Bs (k-major operands) ---
-LNB_DEV void mma_chunk(double (&acc)[2][4][4], const double *as, const double *bs, int wm, int wn, int g, int t)
-{
-#pragma unroll
-    for (int kq = 0; kq < BK / 4; ++kq) {
-        const double *ak = as + (kq * 4 + t) * LDK + wm * 32;
-        const double *bk = bs + (kq * 4 + t) * LDK + wn * 32;
-        double a0[2], a1[2], b0[4];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi) {
-            a0[mi] = ak[mi * 16 + g];
-            a1[mi] = ak[mi * 16 + g + 8];
-        }
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) b0[ni] = bk[ni * 8 + g];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) dmma16x8x4(acc[mi][ni], a0[mi], a1[mi], b0[ni]);
-    }
-}
-
-// stage rows [r0, r0+64) x columns [c0, c0+32) of the column-major matrix as
+// stage rows [r0, r0+64) x columns [c0, c0+16) of the column-major matrix as
 // dst[kk][m] (k-major), rows at or past n zero-filled
 LNB_DEV void stage_chunk(double *dst, const double *A, int64_t lda, int64_t n, int64_t r0, int64_t c0, bool vec,
                          int tid)
 {
     if (vec) {
-        for (int idx = tid; idx < BK * TS / 2; idx += NT) {
-            const int kk = idx / (TS / 2), m2 = (idx % (TS / 2)) * 2;
+#pragma unroll
+        for (int it = 0; it < BK * TS / 2 / NT; ++it) {
+            const int idx = tid + it * NT, kk = idx / (TS / 2), m2 = (idx % (TS / 2)) * 2;
             const int64_t r = r0 + m2;
             const double *g = A + r + (c0 + kk) * lda;
             if (r + 1 < n) {
@@ -250,179 +302,351 @@ LNB_DEV void stage_chunk(double *dst, const double *A, int64_t lda, int64_t n, i
             }
         }
     } else {
-        for (int idx = tid; idx < BK * TS; idx += NT) {
-            const int kk = idx / TS, m = idx % TS;
+#pragma unroll
+        for (int it = 0; it < BK * TS / NT; ++it) {
+            const int idx = tid + it * NT, kk = idx / TS, m = idx % TS;
             const int64_t r = r0 + m;
             cp_async8(dst + kk * LDK + m, r < n ? A + r + (c0 + kk) * lda : A, r < n);
         }
     }
 }
 
-// thread 0 waits for the flags, the CTA learns the outcome (false: give up)
-LNB_DEV bool cta_wait(const int *f0, const int *f1, const Args &a, int site, int item, int *s_ok)
+// at most `left` copy groups of this thread stay in flight (left < ST)
+LNB_DEV void wait_groups(int left)
 {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        bool ok = wait_geq(f0, 1, a.wait_ns, a.st);
-        if (ok && f1 != nullptr) ok = wait_geq(f1, 1, a.wait_ns, a.st);
-        if (!ok && atomicCAS(&a.st->timeout, 0, site) == 0) a.st->timeout_item = item;
-        *s_ok = ok ? 1 : 0;
-    }
-    __syncthreads();
-    return *s_ok != 0;
+    if (left >= 3) cp_async_wait<3>();
+    else if (left == 2) cp_async_wait<2>();
+    else if (left == 1) cp_async_wait<1>();
+    else cp_async_wait<0>();
 }
 
-// fragment (mi, ni, q) of warp (wm, wn) -> tile row / column
-LNB_DEV int frag_row(int wm, int mi, int g, int q) { return wm * 32 + mi * 16 + g + ((q & 2) ? 8 : 0); }
-LNB_DEV int frag_col(int wn, int ni, int t, int q) { return wn * 32 + ni * 8 + 2 * t + (q & 1); }
-
-// one task: produce tile (i, j); false if a wait gave up
-LNB_DEV bool run_tile(const Args &a, int i, int j, double *sm, int *s_ok, int *s_fail)
+// spin until min(*f0, *f1) >= target and return it; -1 after wait_ns or once
+// another waiter has reported a timeout.  hot: a wait on the critical path,
+// without sleeping between the polls.
+LNB_DEV int wait_prog(const int *f0, const int *f1, int target, bool hot, const Args &a)
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp >> 1, wn = warp & 1, g = lane >> 2, t = lane & 3;
-    const int64_t r0 = (int64_t)i * TS, cj = (int64_t)j * TS;
-    const int rows = (int)((a.n - r0) < TS ? (a.n - r0) : TS);       // valid rows of the tile
-    const int cols = (int)((a.n - cj) < TS ? (a.n - cj) : TS);       // valid columns
-    const bool vec = ((uintptr_t)a.A % 16 == 0) && (a.lda % 2 == 0);
-    const int item = j * a.nt + i;
+    const uint64_t t0 = globaltimer();
+    for (int it = 0;; ++it) {
+        int v = ld_acquire(f0);
+        if (f1 != f0 && v >= target) {
+            const int v1 = ld_acquire(f1);
+            v = v1 < v ? v1 : v;
+        }
+        if (v >= target) return v;
+        if ((it & 15) == 15) {
+            if (ld_acquire(&a.st->timeout) != 0) return -1;
+            if ((long long)(globaltimer() - t0) > a.wait_ns) return -1;
+        }
+        if (!hot) __nanosleep(it < 4 ? 64 : 200);
+    }
+}
 
-    // the tile's own entries, loaded early (used after the K loop)
-    double acc[2][4][4], aij[2][4][4];
+LNB_DEV void give_up(const Args &a, int site, int item)
+{
+    if (atomicCAS(&a.st->timeout, 0, site) == 0) a.st->timeout_item = item;
+}
+
+// publish: every thread's stores before the caller's barrier, then one
+// GPU-scope release by one thread
+LNB_DEV void publish(int *flag, int v)
+{
+    __threadfence();
+    asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(flag), "r"(v) : "memory");
+}
+
+// L = S W^T for 16 rows per warp: S k-major in Ss (columns p of S), W^T staged
+// as Ws[p][q] = W[q][p].  W is lower triangular: column block nb needs p < 8 nb + 8.
+LNB_DEV void tile_trsm(double (&o)[8][4], const double *Ss, const double *Ws, int w, int g, int t)
+{
+#pragma unroll
+    for (int nb = 0; nb < 8; ++nb)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) o[nb][q] = 0.0;
+#pragma unroll
+    for (int kq = 0; kq < TS / 4; ++kq) {
+        const double a0 = Ss[(4 * kq + t) * LDK + 16 * w + g], a1 = Ss[(4 * kq + t) * LDK + 16 * w + g + 8];
+#pragma unroll
+        for (int nb = 0; nb < 8; ++nb)
+            if (nb >= kq / 2) dmma16x8x4(o[nb], a0, a1, Ws[(4 * kq + t) * LDK + 8 * nb + g]);
+    }
+}
+
+LNB_DEV void prefetch_l2(const double *p)
+{
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+LNB_DEV int *busy_slot(const Args &a)
+{
+    unsigned smid;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+    return a.busy + (smid & (NBUSY - 1));
+}
+LNB_DEV int ld_relaxed(const int *p)
+{
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// one task: M(j) when i == j, else T(i, j); false if a wait gave up.  Both kinds
+// run the same code: an M task finds the product and TRSM code in its SM's
+// instruction cache.
+LNB_DEV bool run_task(const Args &a, int i, int j, double *sm, Shared &sh)
+{
+    const bool merged = i == j, first = merged && j == 0;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int wm = w >> 1, wn = w & 1, g = lane >> 2, t = lane & 3;
+    const bool vec = ((uintptr_t)a.A % 16 == 0) && (a.lda % 2 == 0);
+    // the product tile: rows of block i, columns of block jc (M: its sub-diagonal tile)
+    const int jc = merged ? (j > 0 ? j - 1 : 0) : j;
+    const int64_t r0 = (int64_t)i * TS, cj = (int64_t)jc * TS;
+    const int rows = (int)((a.n - r0) < TS ? (a.n - r0) : TS);
+    const int item = j * a.nt + i;
+    const bool hot = merged || i == j + 2;
+    const int *pi = a.prog + i, *pj = a.prog + jc;
+
+    // M: the diagonal tile's lower 16 x 8 blocks, five per warp (rows 16 bx, then 16 by)
+    const int bx = w < 2 ? 3 : 2, by = w == 0 ? 3 : w == 1 ? 0 : w == 2 ? 2 : 1;
+    const int nx = w == 1 ? 3 : w == 3 ? 1 : 5, x0 = (w & 1) ? 5 : 0;
+    auto drow = [&](int b) { return 16 * (b < nx ? bx : by); };
+    auto dcol = [&](int b) { return 8 * (b < nx ? x0 + b : b - nx); };
+
+    double acc[2][4][4], dacc[5][4];
+    const int nch = jc * (TS / BK);
+    int issued = 0, known = 0;
+    auto As = [&](int c) { return sm + (c % ST) * 2 * CHUNK; };
+    auto issue = [&](int c) {
+        stage_chunk(As(c), a.A, a.lda, a.n, r0, (int64_t)c * BK, vec, tid);
+        stage_chunk(As(c) + CHUNK, a.A, a.lda, a.n, cj, (int64_t)c * BK, vec, tid);
+        cp_async_commit();
+    };
+
+    if (merged) {                                    // W_j's zeros above the diagonal 16 x 16 blocks
+        double *Wj = a.W + (int64_t)j * TS * TS;
+        for (int q = 16 + (tid >> 3); q < TS; q += NT / 8)
+            for (int r = 2 * (tid & 7); r < (q & ~15); r += 16)
+                *reinterpret_cast<double2 *>(Wj + TS * q + r) = make_double2(0.0, 0.0);
+    }
+    if (merged && j > 0) {
+        // The factor's code runs once per M task, and rarely twice on one SM: a
+        // cold run takes 2.5 times a warm one.  Two panels of an identity tile
+        // fetch it here, ahead of the critical section (W_j gets its own values
+        // before it is published).
+        for (int idx = tid; idx < 3 * PW * LDK; idx += NT) sm[HALF + idx] = idx / LDK == idx % LDK ? 1.0 : 0.0;
+        __syncthreads();
+        cta_factor64(sm + HALF, sm, sm + 2 * HALF, a.W + (int64_t)j * TS * TS, &sh.fail, 3);
+        __syncthreads();
+    }
+    // the tile's own entries are used after the sum (A - sum keeps the rounding
+    // errors at the size of the sum); they come into L2 meanwhile
+    {
+        const int c = tid >> 1;
+        for (int r = 32 * (tid & 1); r < 32 * (tid & 1) + 32 && r < rows; r += 16) {
+            if (!first) prefetch_l2(a.A + (r0 + r) + (cj + c) * a.lda);
+            if (merged && c < rows) prefetch_l2(a.A + (r0 + r) + (r0 + c) * a.lda);
+        }
+    }
 #pragma unroll
     for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
         for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
+            for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
+#pragma unroll
+    for (int b = 0; b < 5; ++b)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dacc[b][q] = 0.0;
+    auto mma_diag = [&](const double *as) {          // dacc += as^T as over BK rows
+#pragma unroll
+        for (int kq = 0; kq < BK / 4; ++kq) {
+            const double *ak = as + (kq * 4 + t) * LDK + g;
+            const double ax0 = ak[16 * bx], ax1 = ak[16 * bx + 8], ay0 = ak[16 * by], ay1 = ak[16 * by + 8];
+#pragma unroll
+            for (int b = 0; b < 5; ++b) dmma16x8x4(dacc[b], b < nx ? ax0 : ay0, b < nx ? ax1 : ay1, ak[dcol(b)]);
+        }
+    };
+
+    // ---- the sums over the finished tiles -------------------------------------
+    // A T task stands back while a task on its SM is in its critical section:
+    // the DMMA pipe is shared, and the factor's dependent chain would queue
+    // behind this task's products.  Only a hint (nothing waits on it), looked
+    // up one chunk ahead and bounded to YIELD_NS.
+    int *const busy = busy_slot(a);
+    int held = 0;
+    for (int kt = 0; kt < nch; ++kt) {
+        const int lim = nch < kt + ST ? nch : kt + ST;
+        if (tid == 0) {
+            if (!merged) {
+                if (held) {
+                    const uint64_t t0 = globaltimer();
+                    while (ld_relaxed(busy) != 0 && globaltimer() - t0 < YIELD_NS) __nanosleep(100);
+                }
+                held = ld_relaxed(busy);
+            }
+            int v = known;
+            const int need = issued / (TS / BK) + 1;
+            if (issued < lim && need > known) {
+                if (issued > kt) {                   // more to do meanwhile: look once
+                    const int v0 = ld_acquire(pi), v1 = ld_acquire(pj);
+                    v = v0 < v1 ? v0 : v1;
+                } else {
+                    v = wait_prog(pi, pj, need, hot, a);
+                    if (v < 0) give_up(a, 31, item);
+                }
+            }
+            sh.known[kt & 1] = v;
+        }
+        const bool had = issued > kt;
+        if (had) wait_groups(issued - kt - 1);
+        __syncthreads();                             // chunk kt is in; its predecessor's slot is free
+        known = sh.known[kt & 1];
+        if (known < 0) {
+            cp_async_wait<0>();
+            return false;
+        }
+        while (issued < lim && issued / (TS / BK) < known) issue(issued++);
+        if (!had) {
+            wait_groups(issued - kt - 1);
+            __syncthreads();
+        }
+        const double *as = As(kt), *bs = as + CHUNK;
+#pragma unroll
+        for (int kq = 0; kq < BK / 4; ++kq) {
+            const double *ak = as + (kq * 4 + t) * LDK + wm * 32 + g, *bk = bs + (kq * 4 + t) * LDK + wn * 32 + g;
+            const double a0[2] = {ak[0], ak[16]}, a1[2] = {ak[8], ak[24]};
+            const double b0[4] = {bk[0], bk[8], bk[16], bk[24]};
+#pragma unroll
+            for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni) dmma16x8x4(acc[mi][ni], a0[mi], a1[mi], b0[ni]);
+        }
+        if (merged) mma_diag(as);
+    }
+    __syncthreads();                                 // the ring is free
+    double *S = sm, *V = sm + HALF;
+
+    if (merged) {
+        // the diagonal tile takes its entries before the last 64 terms (negated)
+#pragma unroll
+        for (int b = 0; b < 5; ++b)
+#pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int r = frag_row(wm, mi, g, q), c = frag_col(wn, ni, t, q);
-                acc[mi][ni][q] = 0.0;
-                aij[mi][ni][q] = (r < rows && c < cols) ? __ldcg(a.A + (r0 + r) + (cj + c) * a.lda) : 0.0;
+                const int r = drow(b) + g + ((q & 2) ? 8 : 0), c = dcol(b) + 2 * t + (q & 1);
+                if (r < rows && r >= c) dacc[b][q] -= __ldcg(a.A + (r0 + r) + (r0 + c) * a.lda);
             }
-
-    // ---- S = A_ij - sum_{k<j} L_ik L_jk^T, two stages of 32-column chunks ----
-    // stage x: A operand at sm + 2 x CHUNK, B operand right after it
-    auto As = [&](int x) { return sm + 2 * x * CHUNK; };
-    auto Bs = [&](int x) { return sm + (2 * x + 1) * CHUNK; };
-    const bool diag = (i == j);
-    const int nch = 2 * j;
-    const int *done_i = a.done + i, *done_j = a.done + j;     // + k * nt
-    if (nch > 0) {
-        if (!cta_wait(done_i, diag ? nullptr : done_j, a, 31, item, s_ok)) return false;
-        stage_chunk(As(0), a.A, a.lda, a.n, r0, 0, vec, tid);
-        if (!diag) stage_chunk(Bs(0), a.A, a.lda, a.n, cj, 0, vec, tid);
-        cp_async_commit();
     }
-    for (int c = 0; c < nch; ++c) {
-        const int nc = c + 1;
-        if (nc < nch) {
-            if ((nc & 1) == 0) {
-                const int k = nc >> 1;
-                // chunk c's data may still be in flight: it stays counted in its group
-                if (!cta_wait(done_i + (int64_t)k * a.nt, diag ? nullptr : done_j + (int64_t)k * a.nt, a, 32,
-                              item, s_ok)) {
-                    cp_async_wait<0>();
-                    return false;
-                }
-            }
-            stage_chunk(As(nc & 1), a.A, a.lda, a.n, r0, (int64_t)nc * BK, vec, tid);
-            if (!diag) stage_chunk(Bs(nc & 1), a.A, a.lda, a.n, cj, (int64_t)nc * BK, vec, tid);
-        }
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        mma_chunk(acc, As(c & 1), diag ? As(c & 1) : Bs(c & 1), wm, wn, g, t);
-        __syncthreads();
-    }
-    cp_async_wait<0>();
-
-    if (diag) {
-        // ---- POTRF of the tile and its inverse ----
-        double *S = sm, *W = sm + TS * LDS;
+    if (!first) {
+        // ---- TRSM: L = S W^T ----
 #pragma unroll
         for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
             for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const int r = frag_row(wm, mi, g, q), c = frag_col(wn, ni, t, q);
-                    // padding past the ragged edge factors as the identity
-                    const double v = (r < rows && c < cols) ? aij[mi][ni][q] - acc[mi][ni][q] : (r == c ? 1.0 : 0.0);
-                    S[r * LDS + c] = v;
+                    const int r = wm * 32 + mi * 16 + g + ((q & 2) ? 8 : 0), c = wn * 32 + ni * 8 + 2 * t + (q & 1);
+                    S[c * LDK + r] =
+                        (r < rows ? __ldcg(a.A + (r0 + r) + (cj + c) * a.lda) : 0.0) - acc[mi][ni][q];
                 }
-        __syncthreads();
-        const int f = cta_potrf64_inv(S, W, s_fail, W + TS * LDS);
-        if (tid == 0 && f < cols) atomicCAS(&a.st->info, 0, (int)(cj + f + 1));
-        // L (lower part, valid rows/columns) and the inverse (whole 64 x 64, column-major)
-        for (int idx = tid; idx < TS * TS; idx += NT) {
-            const int c = idx / TS, r = idx % TS;
-            if (r >= c && r < rows && c < cols) a.A[(cj + r) + (cj + c) * a.lda] = S[r * LDS + c];
-            a.W[(int64_t)j * TS * TS + idx] = W[r * LDS + c];
-        }
-    } else {
-        // ---- TRSM: L_ij = S W_j^T, S staged k-major as the A operand ----
-        if (!cta_wait(a.done + (int64_t)j * a.nt + j, nullptr, a, 33, item, s_ok)) return false;
-        const double *Wj = a.W + (int64_t)j * TS * TS;
-        // W_j^T in two chunks of 32 rows p: B(p, q) = W[q][p] = Wj[q + 64 p], 64 contiguous doubles
-        for (int h = 0; h < 2; ++h)
-            for (int idx = tid; idx < BK * TS / 2; idx += NT) {
-                const int kk = idx / (TS / 2), q2 = (idx % (TS / 2)) * 2;
-                cp_async16(Bs(h) + kk * LDK + q2, Wj + q2 + (int64_t)(h * BK + kk) * TS, true);
+        if (tid == 0) {
+            int v = 0;
+            if (merged) {
+                // tile (jc, jc-1) is published as M(jc) starts its factor: from
+                // there on this task waits for nothing but that factor
+                v = wait_prog(a.prog + jc, a.prog + jc, jc, true, a);
+                atomicAdd(busy, 1);
             }
+            if (v >= 0) v = wait_prog(a.prog + jc, a.prog + jc, jc + 1, hot, a);
+            if (v < 0) give_up(a, 33, item);
+            sh.known[0] = v;
+        }
+        __syncthreads();
+        if (sh.known[0] < 0) return false;
+        const double *Wj = a.W + (int64_t)jc * TS * TS;
+#pragma unroll 8
+        for (int it = 0; it < TS * TS / 2 / NT; ++it) {
+            const int idx = tid + it * NT, kk = idx / (TS / 2), q2 = (idx % (TS / 2)) * 2;
+            cp_async16(V + kk * LDK + q2, Wj + q2 + (int64_t)kk * TS, true);
+        }
         cp_async_commit();
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int r = frag_row(wm, mi, g, q), c = frag_col(wn, ni, t, q);
-                    As(c >> 5)[(c & 31) * LDK + r] = aij[mi][ni][q] - acc[mi][ni][q];
-                    acc[mi][ni][q] = 0.0;
-                }
         cp_async_wait<0>();
         __syncthreads();
-        mma_chunk(acc, As(0), Bs(0), wm, wn, g, t);
-        mma_chunk(acc, As(1), Bs(1), wm, wn, g, t);
+        double o[8][4];
+        tile_trsm(o, S, V, w, g, t);
+        if (merged) {
+            __syncthreads();                         // S is read; L takes its place
 #pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
+            for (int nb = 0; nb < 8; ++nb)
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
+                for (int q = 0; q < 4; ++q)
+                    S[(8 * nb + 2 * t + (q & 1)) * LDK + 16 * w + g + ((q & 2) ? 8 : 0)] = o[nb][q];
+            __syncthreads();
+#pragma unroll 1
+            for (int k0 = 0; k0 < TS; k0 += BK) mma_diag(S + k0 * LDK);
+        }
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int r = frag_row(wm, mi, g, q), c = frag_col(wn, ni, t, q);
-                    if (r < rows && c < cols) a.A[(r0 + r) + (cj + c) * a.lda] = acc[mi][ni][q];
-                }
+        for (int nb = 0; nb < 8; ++nb)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = 16 * w + g + ((q & 2) ? 8 : 0), c = 8 * nb + 2 * t + (q & 1);
+                if (r < rows) a.A[(r0 + r) + (cj + c) * a.lda] = o[nb][q];
+            }
+        if (!merged) {
+            __syncthreads();
+            if (tid == 0) publish(a.prog + i, j + 1);
+        }
     }
-    // publish: every thread's stores, then one GPU-scope release
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        st_release(a.done + (int64_t)j * a.nt + i, 1);
+    if (merged) {
+        // ---- the diagonal tile: S, factor, inverse ----
+#pragma unroll
+        for (int b = 0; b < 5; ++b)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = drow(b) + g + ((q & 2) ? 8 : 0), c = dcol(b) + 2 * t + (q & 1);
+                // padding past the ragged edge factors as the identity
+                V[c * LDK + r] = (r < rows && c < rows) ? -dacc[b][q] : (r == c ? 1.0 : 0.0);
+            }
+        __syncthreads();
+        if (tid == NT - 1 && j > 0) publish(a.prog + j, j);   // tile (j, j-1), off the factor's warp
+        const int f = cta_factor64(V, S, sm + 2 * HALF, a.W + (int64_t)j * TS * TS, &sh.fail, TS / PW);
+        __syncthreads();
+        if (tid == 0) {
+            if (f < rows) atomicCAS(&a.st->info, 0, (int)(r0 + f + 1));
+            publish(a.prog + j, j + 1);
+            if (j > 0) atomicAdd(busy, -1);
+        }
+        // nothing in the walk reads L_jj itself
+        for (int idx = tid; idx < TS * TS; idx += NT) {
+            const int c = idx / TS, r = idx % TS;
+            if (r >= c && r < rows) a.A[(r0 + r) + (r0 + c) * a.lda] = V[c * LDK + r];
+        }
     }
     return true;
 }
 
-__global__ void __launch_bounds__(NT, 2) k_chol_dag_f64(Args a)
+__global__ void __launch_bounds__(NT, 3) k_chol_dag_f64(Args a)
 {
     extern __shared__ __align__(16) double sm[];
-    __shared__ int s_task, s_ok, s_fail[2];
+    __shared__ Shared sh;
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) s_task = atomicAdd(a.ticket, 1) + a.ticket0;
+        if (threadIdx.x == 0) sh.task = atomicAdd(a.ticket, 1) + a.ticket0;
         __syncthreads();
-        const int tk = s_task;
+        const int tk = sh.task;
         if (tk >= a.ntasks) break;
-        // column j holds tickets [j nt - j (j-1)/2, + nt - j): diagonal first, then rows below
-        int lo = 0, hi = a.nt - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            const int64_t start = (int64_t)mid * a.nt - (int64_t)mid * (mid - 1) / 2;
-            if (start <= tk) lo = mid; else hi = mid - 1;
+        int i = tk, j = tk;
+        if (tk >= 2) {
+            // column group c holds tickets [2 + c (nt-1) - c (c-1)/2, + nt - 1 - c)
+            int lo = 0, hi = a.nt - 3;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                const int64_t start = 2 + (int64_t)mid * (a.nt - 1) - (int64_t)mid * (mid - 1) / 2;
+                if (start <= tk) lo = mid; else hi = mid - 1;
+            }
+            const int off = (int)(tk - (2 + (int64_t)lo * (a.nt - 1) - (int64_t)lo * (lo - 1) / 2));
+            i = lo + 2 + (off > 1 ? off - 1 : 0);
+            j = off == 1 ? i : lo;
         }
-        const int j = lo;
-        const int i = j + (int)(tk - ((int64_t)j * a.nt - (int64_t)j * (j - 1) / 2));
-        if (!run_tile(a, i, j, sm, &s_ok, s_fail)) break;
+        if (!run_task(a, i, j, sm, sh)) break;
     }
 }
 
@@ -432,7 +656,7 @@ __global__ void __launch_bounds__(NT, 2) k_chol_dag_f64(Args a)
 extern "C" int64_t lnb_chol_dag_ints(int64_t n)
 {
     const int64_t nt = (n + lnb::dag::TS - 1) / lnb::dag::TS;
-    return nt * nt + 32;
+    return nt + 32 + lnb::dag::NBUSY;
 }
 extern "C" int64_t lnb_chol_dag_w_doubles(int64_t n)
 {
@@ -451,13 +675,13 @@ extern "C" int lnb_k_chol_dag_f64(double *A, int64_t lda, int64_t n, double *W, 
     const int64_t nt = (n + TS - 1) / TS;
     if (nt > 8192) return (int)cudaErrorInvalidValue;
     Args a;
-    a.A = A; a.lda = lda; a.n = n; a.nt = (int)nt; a.ntasks = (int)(nt * (nt + 1) / 2);
-    a.W = W; a.ticket = sync; a.ticket0 = ticket0; a.done = sync + 32; a.st = st; a.wait_ns = wait_ns;
+    a.A = A; a.lda = lda; a.n = n; a.nt = (int)nt; a.ntasks = (int)(1 + nt * (nt - 1) / 2);
+    a.W = W; a.ticket = sync; a.ticket0 = ticket0; a.busy = sync + 32; a.prog = sync + 32 + NBUSY; a.st = st; a.wait_ns = wait_ns;
     cudaError_t e = cudaMemsetAsync(sync, 0, (size_t)lnb_chol_dag_ints(n) * sizeof(int), (cudaStream_t)s);
     if (e != cudaSuccess) return (int)e;
     e = cudaFuncSetAttribute(k_chol_dag_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
-    const int grid = (int)(a.ntasks < 2 * sms ? a.ntasks : 2 * sms);
+    const int grid = (int)(a.ntasks < 3 * sms ? a.ntasks : 3 * sms);
     k_chol_dag_f64<<<grid, NT, SMEM, (cudaStream_t)s>>>(a);
     lnb_prof_count(1);
     return (int)cudaGetLastError();
