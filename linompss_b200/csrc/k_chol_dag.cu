@@ -8,41 +8,54 @@
 // on the GPU:
 //
 //   * The factor is cut into 64 x 64 tiles (the last row and column ragged).
-//     Two kinds of tasks, both left-looking:
+//     Three kinds of tasks, all left-looking:
 //       T(i, j), i >= j + 2:  S = A_ij - sum_{k<j} L_ik L_jk^T,  L_ij = S W_j^T
-//       M(j):  L_{j,j-1} the same way, then
-//              S = A_jj - sum_{k<j} L_jk L_jk^T,  L_jj = potrf(S),  W_j = L_jj^-1
-//     M(j) holds the whole critical path of column j: both tiles accumulate
-//     side by side while column j-1 is being factored, and once W_{j-1} is
-//     there the sub-diagonal tile goes from the TRSM product through shared
-//     memory into the diagonal tile's update and its factor, without a trip
-//     through global memory and a flag in between.
-//   * The sums run in 16-column chunks on DMMA (mma.sync m16n8k4 f64) through a
-//     4-stage cp.async ring, each chunk issued once the two tiles it reads are
-//     final.
+//       P(j), j >= 3:  A_{j,j-1} -= sum_{k<j-2} L_jk L_{j-1,k}^T, in place
+//       M(j):  S = A_jj - sum_{k<j-1} L_jk L_jk^T;  A_{j,j-1} -= the term k = j-2,
+//              L_{j,j-1} = A_{j,j-1} W_{j-1}^T,  S -= L_{j,j-1} L_{j,j-1}^T,
+//              L_jj = potrf(S),  W_j = L_jj^-1
+//     M(j) holds the whole critical path of column j: once W_{j-1} is there the
+//     sub-diagonal tile goes from the TRSM product through shared memory into
+//     the diagonal tile's update and its factor, without a trip through global
+//     memory and a flag in between.  The terms before run ahead of that; P(j)
+//     takes most of them off M(j), which is the longer of the two.
+//   * A CTA is four tensor-core warps (DMMA, mma.sync m16n8k4 f64) and a
+//     producer warp.  The producer polls for the tiles a task reads and brings
+//     16-column chunks of them into a 4-stage ring by cp.async on mbarriers; the
+//     others only load fragments and multiply.  Two CTAs per SM: a third costs
+//     the registers of the multiplying warps (128 instead of 168) and slows the
+//     critical tasks it shares an SM with (n = 16384: 48.6 against 45.2 ms,
+//     n = 2048: 0.57 against 0.48).  With the copies and the polls in the
+//     multiplying warps two CTAs per SM took 65 ms at n = 16384 and three 53.
+//     What bounds it: up to n = 4096 the chain, 13 - 15 us per 64 columns (poll
+//     and W 1.5, TRSM and update 4.1, factor 7.2, publish 0.5); above that the
+//     DMMA rate (30 TF/s at n = 8192, 32.4 at 16384, of 35.4 for cuBLAS dgemm).
 //   * Tasks are handed out by an atomic ticket: M(0), M(1), then per column c
-//     T(c+2, c), M(c+2), T(c+3, c), ...: the device form of the reference's
-//     priorities (the POTRF/TRSM chain goes out two columns ahead of the rest).
-//     A task waits only on tiles with smaller tickets, which running CTAs hold;
-//     so the walk cannot deadlock whatever the residency.
+//     T(c+2, c), P(c+2), M(c+2), T(c+3, c), ...: the device form of the
+//     reference's priorities (the POTRF/TRSM chain goes out two columns ahead of
+//     the rest).  A task waits only on tiles with smaller tickets, which running
+//     CTAs hold; so the walk cannot deadlock whatever the residency.
 //   * The tiles of a row are finished in column order (tile (i, k) needs every
 //     (i, k' < k)), so one counter per row says how many are final.  It is set
-//     by a release of one thread after a CTA barrier and read by an acquire of
-//     one thread before one; a CTA keeps the value it saw and polls again only
-//     past it.  Every wait is bounded by wait_ns of device time; a wait that
-//     runs out sets st->timeout and the CTA drains its copies and stops, and the
-//     other waiters see the timeout and stop too.
+//     by a release of one thread after a barrier of the storing warps and read
+//     by an acquire of the producer's lane 0, which keeps the value it saw and
+//     polls again only past it.  Every wait is bounded by wait_ns of device time;
+//     a wait that runs out sets st->timeout, the CTA's copies land and it stops,
+//     and the other waiters see the timeout and stop too.
 //   * A non-positive pivot is reported LAPACK-style in st->info (1-based
 //     global column); the columns before it are final for every row, and the
 //     walk still finishes every task (with the inverse's rows from the failure
 //     on replaced by identity rows), so nothing waits forever.
 #include "common.cuh"
+#include "tc_sm100.cuh"
 
 namespace lnb {
 namespace dag {
 
 constexpr int TS = 64;              // tile order
-constexpr int NT = 128;             // threads per CTA (4 warps)
+constexpr int NT = 128;             // multiplying threads (4 warps)
+constexpr int NTHR = NT + 32;       // + the producer warp
+constexpr int CPS = 2;              // CTAs per SM
 constexpr int BK = 16;              // K chunk
 constexpr int ST = 4;               // stages of the chunk ring
 constexpr int LDK = TS + 4;         // k-major staged rows (= 4 mod 16 doubles: conflict-free fragments)
@@ -52,8 +65,9 @@ constexpr int PW = 8;               // panel width of the diagonal factor
 constexpr uint64_t YIELD_NS = 40000;
 constexpr int NBUSY = 256;          // SMs told apart by the busy flags
 constexpr int LDX = 10;             // column stride of a panel's 8 x 8 inverse
-static_assert(2 * HALF == 2 * ST * CHUNK, "the epilogue's two tiles fill the ring");
-constexpr int SMEM = (2 * HALF + 2 * PW * LDX) * (int)sizeof(double);
+static_assert(2 * HALF <= 2 * ST * CHUNK, "the epilogue's two tiles fit the ring");
+constexpr int XOFF = 2 * ST * CHUNK;   // the panels' inverses, after the ring
+constexpr int SMEM = (XOFF + 2 * PW * LDX) * (int)sizeof(double);
 
 struct Args {
     double *A;
@@ -61,6 +75,7 @@ struct Args {
     int nt, ntasks;
     double *W;              // nt inverses of the diagonal tiles, 64 x 64 column-major each
     int *prog;              // prog[i]: tiles (i, 0 .. prog[i]-1) are final
+    int *part;              // part[j]: P(j) is done
     int *busy;              // busy[sm]: a task on that SM is in its critical section
     int *ticket;
     int ticket0;            // first ticket handed out (0; 1 only in the wait self-test)
@@ -69,9 +84,32 @@ struct Args {
 };
 
 struct Shared {
+    uint64_t full[ST], empty[ST];   // chunk ring
+    uint64_t kdone;                 // the sums are read: the ring may be overwritten
+    uint64_t sfull, wfull;          // P(j) is done; W is in
     int task, fail;
-    int known[2];
+    int abort;
 };
+// what a CTA has put through its mbarriers so far (every thread keeps the same)
+struct Count {
+    int q, kd, sf, wf;
+};
+
+// barrier of the four multiplying warps
+LNB_DEV void mma_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+LNB_DEV bool mma_sync_and(bool pred)
+{
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, 1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)pred)
+        : "memory");
+    return r != 0;
+}
 
 // 1/sqrt(d) for a normal d > 0: the approximate instruction (relative error
 // 2^-20 measured) and one third-order step of the iteration
@@ -256,7 +294,7 @@ LNB_DEV int cta_factor64(double *Sc, double *Wr, double *Xs2, double *Wg, int *s
                 o1[8] = e3 - (acc[3] + acc2[3]);
             }
         }
-        __syncthreads();                             // panel p is final
+        mma_sync();                                  // panel p is final
         fail = *s_fail;
         if (pn == panels || fail < TS) break;
         if (w >= m0) {                               // panel p's own columns
@@ -272,52 +310,49 @@ LNB_DEV int cta_factor64(double *Sc, double *Wr, double *Xs2, double *Wg, int *s
             o1[8] -= acc[3] + acc2[3];
         }
         if (w <= p / 2) finish_w(p, w);
-        __syncthreads();
+        mma_sync();
     }
     if (w <= p / 2) finish_w(p, w);
     if (fail < TS) {                                 // identity rows from the failure on
-        __syncthreads();
+        mma_sync();
         for (int idx = tid; idx < TS * TS; idx += NT)
             if ((idx & 63) >= fail) Wg[idx] = (idx & 63) == (idx >> 6) ? 1.0 : 0.0;
     }
     return fail;
 }
 
-// stage rows [r0, r0+64) x columns [c0, c0+16) of the column-major matrix as
-// dst[kk][m] (k-major), rows at or past n zero-filled
-LNB_DEV void stage_chunk(double *dst, const double *A, int64_t lda, int64_t n, int64_t r0, int64_t c0, bool vec,
-                         int tid)
+// ---- the producer warp ---------------------------------------------------------
+// rows [r0, r0 + 64) of NC columns from c0 of the column-major matrix as
+// dst[kk][m] (k-major), rows at or past n zero-filled, by cp.async of the warp:
+// 16 bytes per lane where the matrix is 16-byte aligned, else 8.  (A bulk copy
+// per column takes 55 cycles to issue and a proxy fence after each flag; these
+// take 7 and none.)
+template <int NC>
+LNB_DEV void load_cols(double *dst, const double *A, int64_t lda, int64_t n, int64_t r0, int64_t c0, bool vec, int lane)
 {
     if (vec) {
-#pragma unroll
-        for (int it = 0; it < BK * TS / 2 / NT; ++it) {
-            const int idx = tid + it * NT, kk = idx / (TS / 2), m2 = (idx % (TS / 2)) * 2;
-            const int64_t r = r0 + m2;
-            const double *g = A + r + (c0 + kk) * lda;
-            if (r + 1 < n) {
-                cp_async16(dst + kk * LDK + m2, g, true);
-            } else {
-                cp_async8(dst + kk * LDK + m2, r < n ? g : A, r < n);
-                cp_async8(dst + kk * LDK + m2 + 1, A, false);
-            }
-        }
+        const int64_t r = r0 + 2 * lane;
+        const int bytes = r + 1 < n ? 16 : r < n ? 8 : 0;
+        const double *g = A + (bytes ? r : 0) + c0 * lda;
+        uint32_t d = smem_u32(dst + 2 * lane);
+#pragma unroll 8
+        for (int c = 0; c < NC; ++c, g += lda, d += LDK * 8)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(g), "r"(bytes));
     } else {
-#pragma unroll
-        for (int it = 0; it < BK * TS / NT; ++it) {
-            const int idx = tid + it * NT, kk = idx / TS, m = idx % TS;
-            const int64_t r = r0 + m;
-            cp_async8(dst + kk * LDK + m, r < n ? A + r + (c0 + kk) * lda : A, r < n);
+        const int b0 = r0 + lane < n ? 8 : 0, b1 = r0 + lane + 32 < n ? 8 : 0;
+        const double *g0 = A + (b0 ? r0 + lane : 0) + c0 * lda, *g1 = A + (b1 ? r0 + lane + 32 : 0) + c0 * lda;
+        uint32_t d = smem_u32(dst + lane);
+#pragma unroll 8
+        for (int c = 0; c < NC; ++c, g0 += lda, g1 += lda, d += LDK * 8) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(g0), "r"(b0));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d + 256), "l"(g1), "r"(b1));
         }
     }
 }
-
-// at most `left` copy groups of this thread stay in flight (left < ST)
-LNB_DEV void wait_groups(int left)
+// this lane's arrival on bar once its copies so far have landed
+LNB_DEV void arrive_copied(uint64_t *bar)
 {
-    if (left >= 3) cp_async_wait<3>();
-    else if (left == 2) cp_async_wait<2>();
-    else if (left == 1) cp_async_wait<1>();
-    else cp_async_wait<0>();
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // spin until min(*f0, *f1) >= target and return it; -1 after wait_ns or once
@@ -338,6 +373,20 @@ LNB_DEV int wait_prog(const int *f0, const int *f1, int target, bool hot, const 
             if ((long long)(globaltimer() - t0) > a.wait_ns) return -1;
         }
         if (!hot) __nanosleep(it < 4 ? 64 : 200);
+    }
+}
+
+// wait on one of the CTA's mbarriers; false once the CTA has given up or wait_ns
+// has passed.  It polls shared memory only: many CTAs wait at once, and polling
+// the global status word here slowed every flag of the walk down.
+LNB_DEV bool bar_wait(uint64_t *bar, uint32_t parity, long long wait_ns, const Shared &sh)
+{
+    if (tc::mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = globaltimer();
+    for (int it = 1;; ++it) {
+        if (tc::mbar_try_wait(bar, parity)) return true;
+        if (*(const volatile int *)&sh.abort) return false;
+        if ((it & 63) == 0 && (long long)(globaltimer() - t0) > wait_ns) return false;
     }
 }
 
@@ -388,55 +437,120 @@ LNB_DEV int ld_relaxed(const int *p)
     return v;
 }
 
-// one task: M(j) when i == j, else T(i, j); false if a wait gave up.  Both kinds
-// run the same code: an M task finds the product and TRSM code in its SM's
-// instruction cache.
-LNB_DEV bool run_task(const Args &a, int i, int j, double *sm, Shared &sh)
+enum Kind { TASK_T, TASK_P, TASK_M };
+
+// the producer's side of one task; false if a wait gave up
+LNB_DEV bool produce(const Args &a, Kind kind, int i, int j, bool vec, double *sm, Shared &sh, Count &n)
 {
-    const bool merged = i == j, first = merged && j == 0;
+    const int lane = threadIdx.x & 31;
+    const bool merged = kind == TASK_M;
+    if ((merged && j == 0) || (kind == TASK_P && j < 3)) return true;
+    const int jc = kind == TASK_T ? j : j - 1;       // column tile of the product tile
+    const int64_t r0 = (int64_t)i * TS, cj = (int64_t)jc * TS;
+    const int item = j * a.nt + i;
+    const bool hot = kind != TASK_T || i == j + 2;
+    const int *pi = a.prog + i, *pj = a.prog + jc;
+    int *const busy = busy_slot(a);
+    const int nch = (kind == TASK_P ? j - 2 : jc) * (TS / BK);
+    const int both = merged ? nch - TS / BK : 0;     // M reads the column tile's rows in the last term only
+    int known = 0, held = 0;
+    bool ok = true;
+    int c = 0;
+    for (; c < nch && ok; ++c) {
+        // A T task stands back while a task on its SM is in its critical section:
+        // the DMMA pipe is shared, and the factor's dependent chain would queue
+        // behind this task's products.  Only a hint (nothing waits on it), looked
+        // up one chunk ahead and bounded to YIELD_NS.
+        if (kind == TASK_T) {
+            if (lane == 0) {
+                if (held) {
+                    const uint64_t t0 = globaltimer();
+                    while (ld_relaxed(busy) != 0 && globaltimer() - t0 < YIELD_NS) __nanosleep(100);
+                }
+                held = ld_relaxed(busy);
+            }
+            __syncwarp();
+        }
+        if (merged && c == both && j >= 3) {
+            // A_{j,j-1} as P(j) left it
+            int v = 0;
+            if (lane == 0) v = wait_prog(a.part + j, a.part + j, 1, true, a);
+            if (__shfl_sync(0xffffffffu, v, 0) < 0) {
+                ok = false;
+                break;
+            }
+            if (lane == 0) tc::mbar_arrive(&sh.sfull);
+        }
+        if (c / (TS / BK) >= known) {
+            if (lane == 0) known = wait_prog(pi, c < both ? pi : pj, c / (TS / BK) + 1, hot, a);
+            if (c < both && known > both / (TS / BK)) known = both / (TS / BK);
+            known = __shfl_sync(0xffffffffu, known, 0);
+            if (known < 0) {
+                ok = false;
+                break;
+            }
+        }
+        const int s = n.q % ST;
+        if (n.q >= ST && !bar_wait(&sh.empty[s], ((n.q / ST) - 1) & 1, a.wait_ns, sh)) ok = false;
+        if (!__all_sync(0xffffffffu, ok)) {
+            ok = false;
+            break;
+        }
+        double *as = sm + s * 2 * CHUNK;
+        const int64_t c0 = (int64_t)c * BK;
+        load_cols<BK>(as, a.A, a.lda, a.n, r0, c0, vec, lane);
+        if (c >= both) load_cols<BK>(as + CHUNK, a.A, a.lda, a.n, cj, c0, vec, lane);
+        arrive_copied(&sh.full[s]);
+        ++n.q;
+    }
+    if (ok && kind != TASK_P) {
+        double *V = sm + HALF;
+        if (!bar_wait(&sh.kdone, n.kd & 1, 4 * a.wait_ns, sh)) ok = false;
+        ok = __all_sync(0xffffffffu, ok);
+        ++n.kd;
+        if (ok) {
+            int v = 0;
+            if (lane == 0) {
+                if (merged) {
+                    // tile (jc, jc-1) is published as M(jc) starts its factor: from
+                    // there on this task waits for nothing but that factor
+                    v = wait_prog(a.prog + jc, a.prog + jc, jc, true, a);
+                    atomicAdd(busy, 1);
+                }
+                if (v >= 0) v = wait_prog(a.prog + jc, a.prog + jc, jc + 1, hot, a);
+            }
+            v = __shfl_sync(0xffffffffu, v, 0);
+            ok = v >= 0;
+            if (ok) {
+                load_cols<TS>(V, a.W + (int64_t)jc * TS * TS, TS, TS, 0, 0, true, lane);
+                arrive_copied(&sh.wfull);
+                ++n.wf;
+            }
+        }
+    }
+    if (!ok) {
+        if (lane == 0) {
+            give_up(a, 31 + (int)kind, item);
+            sh.abort = 1;
+        }
+        cp_async_wait<0>();
+    }
+    return ok;
+}
+
+// the multiplying warps' side of one task; false if a wait gave up
+LNB_DEV bool multiply(const Args &a, Kind kind, int i, int j, double *sm, Shared &sh, Count &n)
+{
+    const bool merged = kind == TASK_M, first = merged && j == 0;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int wm = w >> 1, wn = w & 1, g = lane >> 2, t = lane & 3;
-    const bool vec = ((uintptr_t)a.A % 16 == 0) && (a.lda % 2 == 0);
-    // the product tile: rows of block i, columns of block jc (M: its sub-diagonal tile)
-    const int jc = merged ? (j > 0 ? j - 1 : 0) : j;
+    const int jc = kind == TASK_T ? j : (j > 0 ? j - 1 : 0);
     const int64_t r0 = (int64_t)i * TS, cj = (int64_t)jc * TS;
     const int rows = (int)((a.n - r0) < TS ? (a.n - r0) : TS);
-    const int item = j * a.nt + i;
-    const bool hot = merged || i == j + 2;
-    const int *pi = a.prog + i, *pj = a.prog + jc;
+    if (kind == TASK_P && j < 3) return true;
+    const int nch = (kind == TASK_P ? j - 2 : jc) * (TS / BK);
+    double *S = sm, *V = sm + HALF;
 
-    // M: the diagonal tile's lower 16 x 8 blocks, five per warp (rows 16 bx, then 16 by)
-    const int bx = w < 2 ? 3 : 2, by = w == 0 ? 3 : w == 1 ? 0 : w == 2 ? 2 : 1;
-    const int nx = w == 1 ? 3 : w == 3 ? 1 : 5, x0 = (w & 1) ? 5 : 0;
-    auto drow = [&](int b) { return 16 * (b < nx ? bx : by); };
-    auto dcol = [&](int b) { return 8 * (b < nx ? x0 + b : b - nx); };
-
-    double acc[2][4][4], dacc[5][4];
-    const int nch = jc * (TS / BK);
-    int issued = 0, known = 0;
-    auto As = [&](int c) { return sm + (c % ST) * 2 * CHUNK; };
-    auto issue = [&](int c) {
-        stage_chunk(As(c), a.A, a.lda, a.n, r0, (int64_t)c * BK, vec, tid);
-        stage_chunk(As(c) + CHUNK, a.A, a.lda, a.n, cj, (int64_t)c * BK, vec, tid);
-        cp_async_commit();
-    };
-
-    if (merged) {                                    // W_j's zeros above the diagonal 16 x 16 blocks
-        double *Wj = a.W + (int64_t)j * TS * TS;
-        for (int q = 16 + (tid >> 3); q < TS; q += NT / 8)
-            for (int r = 2 * (tid & 7); r < (q & ~15); r += 16)
-                *reinterpret_cast<double2 *>(Wj + TS * q + r) = make_double2(0.0, 0.0);
-    }
-    if (merged && j > 0) {
-        // The factor's code runs once per M task, and rarely twice on one SM: a
-        // cold run takes 2.5 times a warm one.  Two panels of an identity tile
-        // fetch it here, ahead of the critical section (W_j gets its own values
-        // before it is published).
-        for (int idx = tid; idx < 3 * PW * LDK; idx += NT) sm[HALF + idx] = idx / LDK == idx % LDK ? 1.0 : 0.0;
-        __syncthreads();
-        cta_factor64(sm + HALF, sm, sm + 2 * HALF, a.W + (int64_t)j * TS * TS, &sh.fail, 3);
-        __syncthreads();
-    }
     // the tile's own entries are used after the sum (A - sum keeps the rounding
     // errors at the size of the sum); they come into L2 meanwhile
     {
@@ -446,16 +560,73 @@ LNB_DEV bool run_task(const Args &a, int i, int j, double *sm, Shared &sh)
             if (merged && c < rows) prefetch_l2(a.A + (r0 + r) + (r0 + c) * a.lda);
         }
     }
+    bool ok = true;
+    auto wait_full = [&](int q) {
+        if (ok && !bar_wait(&sh.full[q % ST], (q / ST) & 1, 4 * a.wait_ns, sh)) ok = false;
+        return ok;
+    };
+
+    double acc[2][4][4];
+    auto product = [&](const double *as) {           // acc += A^T B over BK rows of a ring slot
+        const double *bs = as + CHUNK + t * LDK + g + wn * 32;
+        as += t * LDK + g + wm * 32;
+#pragma unroll
+        for (int kq = 0; kq < BK / 4; ++kq) {
+            const double *ak = as + kq * 4 * LDK, *bk = bs + kq * 4 * LDK;
+            const double a0[2] = {ak[0], ak[16]}, a1[2] = {ak[8], ak[24]};
+            const double b0[4] = {bk[0], bk[8], bk[16], bk[24]};
+#pragma unroll
+            for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni) dmma16x8x4(acc[mi][ni], a0[mi], a1[mi], b0[ni]);
+        }
+    };
+    auto slot = [&](int q) { return sm + (q % ST) * 2 * CHUNK; };
+    auto release = [&]() {
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&sh.empty[n.q % ST]);
+        ++n.q;
+    };
+    // the product tile's entries minus the sum: into S, or back in place.  Sixteen
+    // loads in flight: through one pointer the compiler would finish each
+    // read-modify-write before the next.
+    auto subtract = [&](bool store) {
+#pragma unroll
+        for (int mi = 0; mi < 2; ++mi) {
+            const int r = wm * 32 + mi * 16 + g, c = wn * 32 + 2 * t;
+            double *e = a.A + (r0 + r) + (cj + c) * a.lda;
+            double v[4][4];
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int dr = (q & 2) ? 8 : 0;
+                    v[ni][q] = r + dr < rows ? __ldcg(e + dr + (8 * ni + (q & 1)) * a.lda) : 0.0;
+                }
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int dr = (q & 2) ? 8 : 0;
+                    const double x = v[ni][q] - acc[mi][ni][q];
+                    if (!store) S[(c + 8 * ni + (q & 1)) * LDK + r + dr] = x;
+                    else if (r + dr < rows) e[dr + (8 * ni + (q & 1)) * a.lda] = x;
+                }
+        }
+    };
 #pragma unroll
     for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
         for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
-#pragma unroll
-    for (int b = 0; b < 5; ++b)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dacc[b][q] = 0.0;
+
+    // M: the diagonal tile's lower 16 x 8 blocks, five per warp (rows 16 bx, then 16 by)
+    const int bx = w < 2 ? 3 : 2, by = w == 0 ? 3 : w == 1 ? 0 : w == 2 ? 2 : 1;
+    const int nx = w == 1 ? 3 : w == 3 ? 1 : 5, x0 = (w & 1) ? 5 : 0;
+    auto drow = [&](int b) { return 16 * (b < nx ? bx : by); };
+    auto dcol = [&](int b) { return 8 * (b < nx ? x0 + b : b - nx); };
+    double dacc[5][4];
     auto mma_diag = [&](const double *as) {          // dacc += as^T as over BK rows
 #pragma unroll
         for (int kq = 0; kq < BK / 4; ++kq) {
@@ -465,68 +636,29 @@ LNB_DEV bool run_task(const Args &a, int i, int j, double *sm, Shared &sh)
             for (int b = 0; b < 5; ++b) dmma16x8x4(dacc[b], b < nx ? ax0 : ay0, b < nx ? ax1 : ay1, ak[dcol(b)]);
         }
     };
-
-    // ---- the sums over the finished tiles -------------------------------------
-    // A T task stands back while a task on its SM is in its critical section:
-    // the DMMA pipe is shared, and the factor's dependent chain would queue
-    // behind this task's products.  Only a hint (nothing waits on it), looked
-    // up one chunk ahead and bounded to YIELD_NS.
-    int *const busy = busy_slot(a);
-    int held = 0;
-    for (int kt = 0; kt < nch; ++kt) {
-        const int lim = nch < kt + ST ? nch : kt + ST;
-        if (tid == 0) {
-            if (!merged) {
-                if (held) {
-                    const uint64_t t0 = globaltimer();
-                    while (ld_relaxed(busy) != 0 && globaltimer() - t0 < YIELD_NS) __nanosleep(100);
-                }
-                held = ld_relaxed(busy);
-            }
-            int v = known;
-            const int need = issued / (TS / BK) + 1;
-            if (issued < lim && need > known) {
-                if (issued > kt) {                   // more to do meanwhile: look once
-                    const int v0 = ld_acquire(pi), v1 = ld_acquire(pj);
-                    v = v0 < v1 ? v0 : v1;
-                } else {
-                    v = wait_prog(pi, pj, need, hot, a);
-                    if (v < 0) give_up(a, 31, item);
-                }
-            }
-            sh.known[kt & 1] = v;
+    if (!merged) {
+        for (int c = 0; c < nch; ++c) {
+            if (!wait_full(n.q)) break;
+            product(slot(n.q));
+            release();
         }
-        const bool had = issued > kt;
-        if (had) wait_groups(issued - kt - 1);
-        __syncthreads();                             // chunk kt is in; its predecessor's slot is free
-        known = sh.known[kt & 1];
-        if (known < 0) {
-            cp_async_wait<0>();
-            return false;
-        }
-        while (issued < lim && issued / (TS / BK) < known) issue(issued++);
-        if (!had) {
-            wait_groups(issued - kt - 1);
-            __syncthreads();
-        }
-        const double *as = As(kt), *bs = as + CHUNK;
+    } else {
 #pragma unroll
-        for (int kq = 0; kq < BK / 4; ++kq) {
-            const double *ak = as + (kq * 4 + t) * LDK + wm * 32 + g, *bk = bs + (kq * 4 + t) * LDK + wn * 32 + g;
-            const double a0[2] = {ak[0], ak[16]}, a1[2] = {ak[8], ak[24]};
-            const double b0[4] = {bk[0], bk[8], bk[16], bk[24]};
+        for (int b = 0; b < 5; ++b)
 #pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni) dmma16x8x4(acc[mi][ni], a0[mi], a1[mi], b0[ni]);
+            for (int q = 0; q < 4; ++q) dacc[b][q] = 0.0;
+        const int early = nch - TS / BK;             // chunks before the term k = j-2
+        for (int c = 0; c < early; ++c) {
+            if (!wait_full(n.q)) break;
+            mma_diag(slot(n.q));
+            release();
         }
-        if (merged) mma_diag(as);
-    }
-    __syncthreads();                                 // the ring is free
-    double *S = sm, *V = sm + HALF;
-
-    if (merged) {
-        // the diagonal tile takes its entries before the last 64 terms (negated)
+        // both tiles take their entries before the last 64 terms (negated), the
+        // product tile as P(j) left it
+        if (j >= 3) {
+            if (ok && !bar_wait(&sh.sfull, n.sf & 1, 4 * a.wait_ns, sh)) ok = false;
+            ++n.sf;
+        }
 #pragma unroll
         for (int b = 0; b < 5; ++b)
 #pragma unroll
@@ -534,52 +666,63 @@ LNB_DEV bool run_task(const Args &a, int i, int j, double *sm, Shared &sh)
                 const int r = drow(b) + g + ((q & 2) ? 8 : 0), c = dcol(b) + 2 * t + (q & 1);
                 if (r < rows && r >= c) dacc[b][q] -= __ldcg(a.A + (r0 + r) + (r0 + c) * a.lda);
             }
+        if (!first) {
+#pragma unroll
+            for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int r = wm * 32 + mi * 16 + g + ((q & 2) ? 8 : 0), c = wn * 32 + ni * 8 + 2 * t + (q & 1);
+                        acc[mi][ni][q] = r < rows ? -__ldcg(a.A + (r0 + r) + (cj + c) * a.lda) : 0.0;
+                    }
+            for (int c = early > 0 ? early : 0; c < nch; ++c) {
+                if (!wait_full(n.q)) break;
+                product(slot(n.q));
+                mma_diag(slot(n.q));
+                release();
+            }
+        }
+    }
+    if (!first) {
+        if (kind != TASK_P) {
+            if (lane == 0) tc::mbar_arrive(&sh.kdone);
+            ++n.kd;
+        }
+        if (!mma_sync_and(ok)) return false;         // the ring is free
+        if (merged) {
+#pragma unroll
+            for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        S[(wn * 32 + ni * 8 + 2 * t + (q & 1)) * LDK + wm * 32 + mi * 16 + g + ((q & 2) ? 8 : 0)] =
+                            -acc[mi][ni][q];
+        } else {
+            subtract(kind == TASK_P);
+        }
+        if (kind == TASK_P) {
+            mma_sync();
+            if (tid == 0) publish(a.part + j, 1);
+            return true;
+        }
     }
     if (!first) {
         // ---- TRSM: L = S W^T ----
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int r = wm * 32 + mi * 16 + g + ((q & 2) ? 8 : 0), c = wn * 32 + ni * 8 + 2 * t + (q & 1);
-                    S[c * LDK + r] =
-                        (r < rows ? __ldcg(a.A + (r0 + r) + (cj + c) * a.lda) : 0.0) - acc[mi][ni][q];
-                }
-        if (tid == 0) {
-            int v = 0;
-            if (merged) {
-                // tile (jc, jc-1) is published as M(jc) starts its factor: from
-                // there on this task waits for nothing but that factor
-                v = wait_prog(a.prog + jc, a.prog + jc, jc, true, a);
-                atomicAdd(busy, 1);
-            }
-            if (v >= 0) v = wait_prog(a.prog + jc, a.prog + jc, jc + 1, hot, a);
-            if (v < 0) give_up(a, 33, item);
-            sh.known[0] = v;
-        }
-        __syncthreads();
-        if (sh.known[0] < 0) return false;
-        const double *Wj = a.W + (int64_t)jc * TS * TS;
-#pragma unroll 8
-        for (int it = 0; it < TS * TS / 2 / NT; ++it) {
-            const int idx = tid + it * NT, kk = idx / (TS / 2), q2 = (idx % (TS / 2)) * 2;
-            cp_async16(V + kk * LDK + q2, Wj + q2 + (int64_t)kk * TS, true);
-        }
-        cp_async_commit();
-        cp_async_wait<0>();
-        __syncthreads();
+        if (ok && !bar_wait(&sh.wfull, n.wf & 1, 4 * a.wait_ns, sh)) ok = false;
+        ++n.wf;
+        if (!mma_sync_and(ok)) return false;
         double o[8][4];
         tile_trsm(o, S, V, w, g, t);
         if (merged) {
-            __syncthreads();                         // S is read; L takes its place
+            mma_sync();                              // S is read; L takes its place
 #pragma unroll
             for (int nb = 0; nb < 8; ++nb)
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
                     S[(8 * nb + 2 * t + (q & 1)) * LDK + 16 * w + g + ((q & 2) ? 8 : 0)] = o[nb][q];
-            __syncthreads();
+            mma_sync();
 #pragma unroll 1
             for (int k0 = 0; k0 < TS; k0 += BK) mma_diag(S + k0 * LDK);
         }
@@ -591,7 +734,7 @@ LNB_DEV bool run_task(const Args &a, int i, int j, double *sm, Shared &sh)
                 if (r < rows) a.A[(r0 + r) + (cj + c) * a.lda] = o[nb][q];
             }
         if (!merged) {
-            __syncthreads();
+            mma_sync();
             if (tid == 0) publish(a.prog + i, j + 1);
         }
     }
@@ -605,14 +748,14 @@ LNB_DEV bool run_task(const Args &a, int i, int j, double *sm, Shared &sh)
                 // padding past the ragged edge factors as the identity
                 V[c * LDK + r] = (r < rows && c < rows) ? -dacc[b][q] : (r == c ? 1.0 : 0.0);
             }
-        __syncthreads();
+        mma_sync();
         if (tid == NT - 1 && j > 0) publish(a.prog + j, j);   // tile (j, j-1), off the factor's warp
-        const int f = cta_factor64(V, S, sm + 2 * HALF, a.W + (int64_t)j * TS * TS, &sh.fail, TS / PW);
-        __syncthreads();
+        const int f = cta_factor64(V, S, sm + XOFF, a.W + (int64_t)j * TS * TS, &sh.fail, TS / PW);
+        mma_sync();
         if (tid == 0) {
             if (f < rows) atomicCAS(&a.st->info, 0, (int)(r0 + f + 1));
             publish(a.prog + j, j + 1);
-            if (j > 0) atomicAdd(busy, -1);
+            if (j > 0) atomicAdd(busy_slot(a), -1);
         }
         // nothing in the walk reads L_jj itself
         for (int idx = tid; idx < TS * TS; idx += NT) {
@@ -623,30 +766,70 @@ LNB_DEV bool run_task(const Args &a, int i, int j, double *sm, Shared &sh)
     return true;
 }
 
-__global__ void __launch_bounds__(NT, 3) k_chol_dag_f64(Args a)
+// before an M task: W_j's zeros above the diagonal 16 x 16 blocks; and the
+// factor's code, which runs once per M task and rarely twice on one SM (a cold
+// run took 2.5 times a warm one), is fetched by three panels of an identity
+// tile, ahead of the critical section (W_j gets its own values before it is
+// published)
+LNB_DEV void warm_factor(const Args &a, int j, double *sm, Shared &sh)
 {
-    extern __shared__ __align__(16) double sm[];
-    __shared__ Shared sh;
+    const int tid = threadIdx.x;
+    double *Wj = a.W + (int64_t)j * TS * TS;
+    for (int q = 16 + (tid >> 3); q < TS; q += NT / 8)
+        for (int r = 2 * (tid & 7); r < (q & ~15); r += 16)
+            *reinterpret_cast<double2 *>(Wj + TS * q + r) = make_double2(0.0, 0.0);
+    if (j == 0) return;
+    for (int idx = tid; idx < 3 * PW * LDK; idx += NT) sm[HALF + idx] = idx / LDK == idx % LDK ? 1.0 : 0.0;
+    mma_sync();
+    cta_factor64(sm + HALF, sm, sm + XOFF, Wj, &sh.fail, 3);
+}
+
+__global__ void __launch_bounds__(NTHR, CPS) k_chol_dag_f64(Args a)
+{
+    extern __shared__ __align__(128) double sm[];
+    __shared__ __align__(8) Shared sh;
+    const bool vec = ((uintptr_t)a.A % 16 == 0) && (a.lda % 2 == 0);
+    const int warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < ST; ++s) {
+            tc::mbar_init(&sh.full[s], 32);
+            tc::mbar_init(&sh.empty[s], NT / 32);
+        }
+        tc::mbar_init(&sh.kdone, NT / 32);
+        tc::mbar_init(&sh.sfull, 1);
+        tc::mbar_init(&sh.wfull, 32);
+        sh.abort = 0;
+        tc::fence_mbar_init();
+    }
+    Count n = {0, 0, 0, 0};
     for (;;) {
         __syncthreads();
+        if (*(volatile int *)&sh.abort) break;       // the same for every thread: set before the barrier
         if (threadIdx.x == 0) sh.task = atomicAdd(a.ticket, 1) + a.ticket0;
         __syncthreads();
         const int tk = sh.task;
         if (tk >= a.ntasks) break;
         int i = tk, j = tk;
+        Kind kind = TASK_M;
         if (tk >= 2) {
-            // column group c holds tickets [2 + c (nt-1) - c (c-1)/2, + nt - 1 - c)
+            // column group c holds tickets [2 + c nt - c (c-1)/2, + nt - c)
             int lo = 0, hi = a.nt - 3;
             while (lo < hi) {
                 const int mid = (lo + hi + 1) >> 1;
-                const int64_t start = 2 + (int64_t)mid * (a.nt - 1) - (int64_t)mid * (mid - 1) / 2;
+                const int64_t start = 2 + (int64_t)mid * a.nt - (int64_t)mid * (mid - 1) / 2;
                 if (start <= tk) lo = mid; else hi = mid - 1;
             }
-            const int off = (int)(tk - (2 + (int64_t)lo * (a.nt - 1) - (int64_t)lo * (lo - 1) / 2));
-            i = lo + 2 + (off > 1 ? off - 1 : 0);
-            j = off == 1 ? i : lo;
+            const int off = (int)(tk - (2 + (int64_t)lo * a.nt - (int64_t)lo * (lo - 1) / 2));
+            kind = off == 1 ? TASK_P : off == 2 ? TASK_M : TASK_T;
+            i = lo + 2 + (off > 2 ? off - 2 : 0);
+            j = kind == TASK_T ? lo : i;
         }
-        if (!run_task(a, i, j, sm, sh)) break;
+        if (kind == TASK_M) {
+            if (warp < NT / 32) warm_factor(a, j, sm, sh);
+            __syncthreads();                         // before the producer's copies
+        }
+        if (warp == NT / 32 ? !produce(a, kind, i, j, vec, sm, sh, n) : !multiply(a, kind, i, j, sm, sh, n))
+            sh.abort = 1;
     }
 }
 
@@ -656,7 +839,7 @@ __global__ void __launch_bounds__(NT, 3) k_chol_dag_f64(Args a)
 extern "C" int64_t lnb_chol_dag_ints(int64_t n)
 {
     const int64_t nt = (n + lnb::dag::TS - 1) / lnb::dag::TS;
-    return nt + 32 + lnb::dag::NBUSY;
+    return 2 * nt + 32 + lnb::dag::NBUSY;
 }
 extern "C" int64_t lnb_chol_dag_w_doubles(int64_t n)
 {
@@ -675,14 +858,14 @@ extern "C" int lnb_k_chol_dag_f64(double *A, int64_t lda, int64_t n, double *W, 
     const int64_t nt = (n + TS - 1) / TS;
     if (nt > 8192) return (int)cudaErrorInvalidValue;
     Args a;
-    a.A = A; a.lda = lda; a.n = n; a.nt = (int)nt; a.ntasks = (int)(1 + nt * (nt - 1) / 2);
-    a.W = W; a.ticket = sync; a.ticket0 = ticket0; a.busy = sync + 32; a.prog = sync + 32 + NBUSY; a.st = st; a.wait_ns = wait_ns;
+    a.A = A; a.lda = lda; a.n = n; a.nt = (int)nt; a.ntasks = (int)(nt < 2 ? nt : 2 + (nt - 2) * (nt + 3) / 2);
+    a.W = W; a.ticket = sync; a.ticket0 = ticket0; a.busy = sync + 32; a.prog = sync + 32 + NBUSY; a.part = a.prog + nt; a.st = st; a.wait_ns = wait_ns;
     cudaError_t e = cudaMemsetAsync(sync, 0, (size_t)lnb_chol_dag_ints(n) * sizeof(int), (cudaStream_t)s);
     if (e != cudaSuccess) return (int)e;
     e = cudaFuncSetAttribute(k_chol_dag_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
-    const int grid = (int)(a.ntasks < 3 * sms ? a.ntasks : 3 * sms);
-    k_chol_dag_f64<<<grid, NT, SMEM, (cudaStream_t)s>>>(a);
+    const int grid = (int)(a.ntasks < CPS * sms ? a.ntasks : CPS * sms);
+    k_chol_dag_f64<<<grid, NTHR, SMEM, (cudaStream_t)s>>>(a);
     lnb_prof_count(1);
     return (int)cudaGetLastError();
 }
