@@ -8,14 +8,15 @@
  * The reference factors b-wide panels with LAPACK dgetrf over every row below
  * (so its pivots are LAPACK's), then swaps the other block columns and updates
  * those on the right with a unit-lower TRSM and a GEMM.  Here the same
- * factorization is blocked for the GPU at two levels:
- *   * outer blocks of 256 columns: once a block is factored, its swaps go to
- *     every other column, its rows of U come from one blocked TRSM
+ * factorization is blocked for the GPU:
+ *   * panels of up to 16 columns are factored by one CTA or a cluster (k_lu.cu),
+ *     and one more launch gives the other columns the panel's swaps, its rows of
+ *     U and its update;
+ *   * while the matrix fits half of the L2 cache that is all; above, this happens
+ *     inside outer blocks of 256 columns: once a block is factored, its swaps go
+ *     to every other column, its rows of U come from one blocked TRSM
  *     (lnb_trsm_f64_run, unit lower), and the rest of the matrix takes one
- *     DMMA GEMM of depth 256;
- *   * inside a block, panels of up to 32 columns are factored in shared memory
- *     by one thread-block cluster (k_lu.cu), and the block's remaining columns
- *     take the panel's swaps, a small unit-lower solve and a GEMM.
+ *     DMMA GEMM of depth 256.
  * Partial pivoting over all rows below gives LAPACK's pivot sequence whatever
  * the blocking, so the user's b only shapes the pivot indices returned: the
  * reference leaves each b-wide panel's pivots as dgetrf returned them for the
@@ -37,17 +38,34 @@
     } while (0)
 
 #define LU_BO 256
+/* up to this many elements (64 MB, half the L2 cache) every panel updates all
+ * the columns right of it: the rank-16 passes over the matrix stay in L2 */
+#define LU_ONE_LEVEL (8LL << 20)
 
 int lnb_lu_panel_width(int64_t rows);
-int lnb_k_lu_panel_f64(double *A, int64_t lda, int64_t m, int64_t c0, int nb, int *piv, lnb_status_t *st,
-                       cudaStream_t s);
+size_t lnb_lu_perm_bytes(void);
+int lnb_k_lu_panel_f64(double *A, int64_t lda, int64_t m, int64_t c0, int nb, int *piv, void *perm,
+                       lnb_status_t *st, cudaStream_t s);
+int lnb_k_lu_apply_f64(double *A, int64_t lda, int64_t m, int64_t c0, int nb, const void *perm, int64_t a0,
+                       int64_t a1, int64_t b0, int64_t b1, cudaStream_t s);
 int lnb_k_laswp_f64(double *A, int64_t lda, int64_t k0, int64_t k1, const int *piv, int64_t a0, int64_t a1,
                     int64_t b0, int64_t b1, cudaStream_t s);
-int lnb_k_lu_trsm_unit_f64(double *A, int64_t lda, int64_t c0, int nb, int64_t j0, int64_t j1, cudaStream_t s);
+int lnb_k_rows_permute_f64(double *B, int64_t ldb, int64_t n, int64_t nrhs, int64_t k1, const int *piv, int *src,
+                           double *T, cudaStream_t s);
 int lnb_k_f32_to_f64(const float *X, int64_t ldx, int64_t m, int64_t k, double *D, int64_t ldd, cudaStream_t st);
 int lnb_k_f64_to_f32(const double *D, int64_t ldd, int64_t m, int64_t k, float *X, int64_t ldx, cudaStream_t st);
 
-static size_t getrf_ws_bytes(int64_t n) { return lnb_trsm_f64_ws_bytes(LU_BO, n) + 1024; }
+static size_t getrf_ws_bytes(int64_t n)
+{
+    return lnb_align256(lnb_lu_perm_bytes()) + lnb_trsm_f64_ws_bytes(LU_BO, n) + 1024;
+}
+
+static size_t getrs_ws_bytes(int64_t n, int64_t nrhs)
+{
+    const size_t t = lnb_trsm_f64_ws_bytes(n, nrhs) + 1024;
+    const size_t p = lnb_align256((size_t)n * 4) + lnb_align256((size_t)n * nrhs * 8);
+    return t > p ? t : p;
+}
 
 /* P A = L U of dA (m x n) in place; dpiv: min(m, n) LAPACK pivots (1-based,
  * global rows).  An exactly zero pivot sets st->info (its 1-based column). */
@@ -58,25 +76,25 @@ static int getrf_run(lnb_ctx *c, int64_t m, int64_t n, double *dA, int64_t lda, 
     if (mn <= 0) return 0;
     if (!lnb_lu_panel_width(m))
         return lnb_set_error(LNB_ETOOBIG, "getrf: %lld rows exceed a panel cluster's shared memory", (long long)m);
-    for (int64_t o0 = 0; o0 < mn; o0 += LU_BO) {
-        const int64_t ob = mn - o0 < LU_BO ? mn - o0 : LU_BO, oe = o0 + ob;
+    lnb_arena a1 = *ar;
+    void *perm = lnb_arena_take(&a1, lnb_lu_perm_bytes());
+    if (!perm) return lnb_set_error(LNB_ENOMEM, "getrf workspace");
+    const int64_t bo = m * n <= LU_ONE_LEVEL ? mn : LU_BO;
+    for (int64_t o0 = 0; o0 < mn; o0 += bo) {
+        const int64_t ob = mn - o0 < bo ? mn - o0 : bo, oe = o0 + ob;
+        /* the block's own columns; all of them in the one-level form */
+        const int64_t cl = bo == mn ? 0 : o0, cr = bo == mn ? n : oe;
         for (int64_t c0 = o0; c0 < oe;) {
             int nb = lnb_lu_panel_width(m - c0);
             if (nb > oe - c0) nb = (int)(oe - c0);
-            CK(lnb_k_lu_panel_f64(dA, lda, m, c0, nb, dpiv, c->st, s), "lu panel");
-            CK(lnb_k_laswp_f64(dA, lda, c0, c0 + nb, dpiv, o0, c0, c0 + nb, oe, s), "panel swaps");
-            if (c0 + nb < oe) {
-                CK(lnb_k_lu_trsm_unit_f64(dA, lda, c0, nb, c0 + nb, oe, s), "panel solve");
-                if (m > c0 + nb)
-                    CK(lnb_k_gemm_tri_f64('N', 'N', m - c0 - nb, oe - c0 - nb, nb, -1.0, dA + (c0 + nb) + c0 * lda,
-                                          lda, dA + c0 + (c0 + nb) * lda, lda, 1.0,
-                                          dA + (c0 + nb) + (c0 + nb) * lda, lda, 0, s), "panel update");
-            }
+            CK(lnb_k_lu_panel_f64(dA, lda, m, c0, nb, dpiv, perm, c->st, s), "lu panel");
+            CK(lnb_k_lu_apply_f64(dA, lda, m, c0, nb, perm, cl, c0, c0 + nb, cr, s), "panel update");
             c0 += nb;
         }
+        if (bo == mn) break;
         CK(lnb_k_laswp_f64(dA, lda, o0, oe, dpiv, 0, o0, oe, n, s), "block swaps");
         if (oe < n) {
-            lnb_arena a2 = *ar;
+            lnb_arena a2 = a1;
             const int e = lnb_trsm_f64_run(c, 'L', 'N', 'U', ob, n - oe, 1.0, dA + o0 + o0 * lda, lda,
                                            dA + o0 + oe * lda, lda, &a2, s, NULL);
             if (e) return e;
@@ -94,8 +112,12 @@ static int getrs_run(lnb_ctx *c, int64_t n, int64_t nrhs, const double *dLU, int
                      double *dB, int64_t ldb, lnb_arena *ar, cudaStream_t s)
 {
     if (n <= 0 || nrhs <= 0) return 0;
-    CK(lnb_k_laswp_f64(dB, ldb, 0, n, dpiv, 0, nrhs, 0, 0, s), "rhs swaps");
     lnb_arena a2 = *ar;
+    int *src = lnb_arena_take(&a2, (size_t)n * 4);
+    double *T = lnb_arena_take(&a2, (size_t)n * nrhs * 8);
+    if (!src || !T) return lnb_set_error(LNB_ENOMEM, "getrs workspace");
+    CK(lnb_k_rows_permute_f64(dB, ldb, n, nrhs, n, dpiv, src, T, s), "rhs swaps");
+    a2 = *ar;
     int e = lnb_trsm_f64_run(c, 'L', 'N', 'U', n, nrhs, 1.0, dLU, lda, dB, ldb, &a2, s, NULL);
     if (e) return e;
     a2 = *ar;
@@ -188,7 +210,7 @@ static int gensolv_host(int m, int n, int b, void *A, void *B, int single)
     const int64_t ldd = ld_dev(m);
     const size_t abytes = (size_t)ldd * m * 8, bbytes = (size_t)ldd * (n ? n : 1) * 8, pbytes = (size_t)m * 4;
     const size_t fbytes = single ? (size_t)m * (m > n ? m : n) * 4 : 0;
-    const size_t w1 = getrf_ws_bytes(m), w2 = lnb_trsm_f64_ws_bytes(m, n) + 1024;
+    const size_t w1 = getrf_ws_bytes(m), w2 = getrs_ws_bytes(m, n);
     void *ws = lnb_ws(c, lnb_align256(abytes) + lnb_align256(bbytes) + lnb_align256(pbytes) + lnb_align256(fbytes) +
                              (w1 > w2 ? w1 : w2));
     if (!ws) return LNB_ENOMEM;
@@ -240,7 +262,7 @@ int lnb_dgetrs_dev(int n, int nrhs, const double *dLU, int lda, const int *dipiv
     if (!dLU || !dipiv || !dB) return lnb_set_error(LNB_EINVAL, "getrs: NULL argument");
     lnb_ctx *c = lnb_ctx_get();
     if (!c) return LNB_ENODEV;
-    void *ws = lnb_ws(c, lnb_trsm_f64_ws_bytes(n, nrhs) + 1024);
+    void *ws = lnb_ws(c, getrs_ws_bytes(n, nrhs) + 1024);
     if (!ws) return LNB_ENOMEM;
     lnb_arena ar = {(char *)ws, 0, c->ws_size};
     return getrs_run(c, n, nrhs, dLU, lda, dipiv, dB, ldb, &ar, (cudaStream_t)stream);
