@@ -626,7 +626,7 @@ LNB_DEV bool multiply(const Args &a, Kind kind, int i, int j, double *sm, Shared
     const int nx = w == 1 ? 3 : w == 3 ? 1 : 5, x0 = (w & 1) ? 5 : 0;
     auto drow = [&](int b) { return 16 * (b < nx ? bx : by); };
     auto dcol = [&](int b) { return 8 * (b < nx ? x0 + b : b - nx); };
-    double dacc[5][4];
+    double dacc[5][4], da[5][4];                     // its sum, its entries
     auto mma_diag = [&](const double *as) {          // dacc += as^T as over BK rows
 #pragma unroll
         for (int kq = 0; kq < BK / 4; ++kq) {
@@ -653,36 +653,23 @@ LNB_DEV bool multiply(const Args &a, Kind kind, int i, int j, double *sm, Shared
             mma_diag(slot(n.q));
             release();
         }
-        // both tiles take their entries before the last 64 terms (negated), the
-        // product tile as P(j) left it
-        if (j >= 3) {
+        if (j >= 3) {                                // the product tile is as P(j) left it
             if (ok && !bar_wait(&sh.sfull, n.sf & 1, 4 * a.wait_ns, sh)) ok = false;
             ++n.sf;
+        }
+        for (int c = early > 0 ? early : 0; c < nch; ++c) {
+            if (!wait_full(n.q)) break;
+            product(slot(n.q));
+            mma_diag(slot(n.q));
+            release();
         }
 #pragma unroll
         for (int b = 0; b < 5; ++b)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int r = drow(b) + g + ((q & 2) ? 8 : 0), c = dcol(b) + 2 * t + (q & 1);
-                if (r < rows && r >= c) dacc[b][q] -= __ldcg(a.A + (r0 + r) + (r0 + c) * a.lda);
+                da[b][q] = r < rows && r >= c ? __ldcg(a.A + (r0 + r) + (r0 + c) * a.lda) : 0.0;
             }
-        if (!first) {
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int r = wm * 32 + mi * 16 + g + ((q & 2) ? 8 : 0), c = wn * 32 + ni * 8 + 2 * t + (q & 1);
-                        acc[mi][ni][q] = r < rows ? -__ldcg(a.A + (r0 + r) + (cj + c) * a.lda) : 0.0;
-                    }
-            for (int c = early > 0 ? early : 0; c < nch; ++c) {
-                if (!wait_full(n.q)) break;
-                product(slot(n.q));
-                mma_diag(slot(n.q));
-                release();
-            }
-        }
     }
     if (!first) {
         if (kind != TASK_P) {
@@ -690,18 +677,7 @@ LNB_DEV bool multiply(const Args &a, Kind kind, int i, int j, double *sm, Shared
             ++n.kd;
         }
         if (!mma_sync_and(ok)) return false;         // the ring is free
-        if (merged) {
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        S[(wn * 32 + ni * 8 + 2 * t + (q & 1)) * LDK + wm * 32 + mi * 16 + g + ((q & 2) ? 8 : 0)] =
-                            -acc[mi][ni][q];
-        } else {
-            subtract(kind == TASK_P);
-        }
+        subtract(kind == TASK_P);
         if (kind == TASK_P) {
             mma_sync();
             if (tid == 0) publish(a.part + j, 1);
@@ -746,7 +722,7 @@ LNB_DEV bool multiply(const Args &a, Kind kind, int i, int j, double *sm, Shared
             for (int q = 0; q < 4; ++q) {
                 const int r = drow(b) + g + ((q & 2) ? 8 : 0), c = dcol(b) + 2 * t + (q & 1);
                 // padding past the ragged edge factors as the identity
-                V[c * LDK + r] = (r < rows && c < rows) ? -dacc[b][q] : (r == c ? 1.0 : 0.0);
+                V[c * LDK + r] = (r < rows && c < rows) ? da[b][q] - dacc[b][q] : (r == c ? 1.0 : 0.0);
             }
         mma_sync();
         if (tid == NT - 1 && j > 0) publish(a.prog + j, j);   // tile (j, j-1), off the factor's warp

@@ -1,4 +1,6 @@
-// k_trsv.cu -- blocked triangular solves with many or few right-hand sides.
+// k_trsv.cu -- inverses of diagonal blocks, and blocked triangular solves with an
+// FP32 factor and many right-hand sides (k_trsv_chain.cu: few; FP64 factors:
+// k_trsm_tiles.cu).
 //
 // Semantics of bblas_dltrsm (bblas_trsm.h:116-202) and of the two solves of
 // dspdsolv_main (spdsolv_main.c:15,17): op(T) X = alpha B with T triangular.
@@ -30,46 +32,93 @@ constexpr int NRC = 64;         // rhs columns per pass
 // ------------------------------------------------------------------------
 // inverses of the diagonal blocks
 // ------------------------------------------------------------------------
-// the inverses are computed in FP64 and stored in the precision of T
+// One CTA inverts one 64 x 64 block, in FP64, stored in the precision of T.  An
+// upper block is inverted as the transpose of its transpose.  The four 16 x 16
+// diagonal blocks by forward substitution (a thread per column), then twice the
+// two-by-two step [A 0; C D]^-1 = [A^-1 0; -D^-1 C A^-1  D^-1], 16 -> 32 -> 64.
+// Bound by latency: the substitution over all 64 rows, a thread per column, was
+// 64 dependent rows of up to 64 terms and took 56 us; this takes 6.
+constexpr int TI_NT = 256, TI_LD = TH + 1;
+// Z (h x h) = sum_k X[.][k] Y[k][.] of h x h blocks (row-major, ld TI_LD), sign s;
+// `part` of the CTA's threads: np threads, this one is p
+LNB_DEV void ti_product(double *Z, const double *X, const double *Y, int h, double s, int p, int np)
+{
+    for (int idx = 4 * p; idx < h * h; idx += 4 * np) {
+        const int r = idx / h, c = idx % h;
+        double z0 = 0.0, z1 = 0.0, z2 = 0.0, z3 = 0.0;
+#pragma unroll 8
+        for (int k = 0; k < h; ++k) {
+            const double x = X[r * TI_LD + k];
+            const double *y = Y + k * TI_LD + c;
+            z0 = fma(x, y[0], z0);
+            z1 = fma(x, y[1], z1);
+            z2 = fma(x, y[2], z2);
+            z3 = fma(x, y[3], z3);
+        }
+        double *z = Z + r * TI_LD + c;
+        z[0] = s * z0;
+        z[1] = s * z1;
+        z[2] = s * z2;
+        z[3] = s * z3;
+    }
+}
 template <typename TT>
-__global__ void __launch_bounds__(TH) k_trtri_blocks(const TT *T, int64_t ldt, int64_t n, char uplo, int unit,
-                                                     TT *dinv)
+__global__ void __launch_bounds__(TI_NT) k_trtri_blocks(const TT *T, int64_t ldt, int64_t n, char uplo, int unit,
+                                                        TT *dinv)
 {
     extern __shared__ double smx[];
-    double (*X)[TH + 1] = reinterpret_cast<double (*)[TH + 1]>(smx);              // X[r][c], column c owned by thread c
-    double (*Tb)[TH + 1] = reinterpret_cast<double (*)[TH + 1]>(smx + TH * (TH + 1));
-    const int q = blockIdx.x, c = threadIdx.x;
+    double *L = smx, *X = smx + TH * TI_LD;        // row-major: the block (lower), its inverse
+    const int q = blockIdx.x, tid = threadIdx.x;
     const int64_t o = (int64_t)q * TH;
     const int qn = (int)((n - o) < TH ? (n - o) : TH);
-    for (int r = 0; r < TH; ++r) {
-        double v = 0.0;
-        if (r < qn && c < qn) v = (double)T[(o + r) + (o + c) * ldt];
-        Tb[r][c] = v;
+    const bool lower = uplo == 'L';
+    // padding past the ragged edge inverts as the identity
+    for (int idx = tid; idx < TH * TH; idx += TI_NT) {
+        const int c = idx / TH, r = idx % TH;      // stored row r, column c
+        double v = r == c ? 1.0 : 0.0;
+        if (r < qn && c < qn && (lower ? r >= c : r <= c) && !(unit && r == c)) v = (double)T[(o + r) + (o + c) * ldt];
+        L[lower ? r * TI_LD + c : c * TI_LD + r] = v;
+        X[r * TI_LD + c] = 0.0;
     }
     __syncthreads();
-    for (int r = 0; r < TH; ++r) X[r][c] = 0.0;
-    if (c >= qn) {
-        X[c][c] = 1.0;
-    } else if (uplo == 'L') {
-        // column c of inv(L): x[c] = 1/L[c][c]; x[r] = -(sum_{p=c}^{r-1} L[r][p] x[p]) / L[r][r]
-        X[c][c] = unit ? 1.0 : 1.0 / Tb[c][c];
-        for (int r = c + 1; r < qn; ++r) {
-            double s = 0.0;
-            for (int p = c; p < r; ++p) s += Tb[r][p] * X[p][c];
-            X[r][c] = unit ? -s : -s / Tb[r][r];
+    if (tid < TH) {
+        const int b0 = tid & ~15, c = tid & 15;    // column c of the 16 x 16 block at b0
+        const double *Lb = L + b0 * TI_LD + b0;
+        double x[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            double s = r == c ? 1.0 : 0.0, s2 = 0.0;
+#pragma unroll
+            for (int p = 0; p < r; ++p) {
+                if (p & 1) s2 = fma(-Lb[r * TI_LD + p], x[p], s2);
+                else s = fma(-Lb[r * TI_LD + p], x[p], s);
+            }
+            x[r] = (s + s2) / Lb[r * TI_LD + r];
         }
-    } else {
-        // column c of inv(U): x[c] = 1/U[c][c]; x[r] = -(sum_{p=r+1}^{c} U[r][p] x[p]) / U[r][r]
-        X[c][c] = unit ? 1.0 : 1.0 / Tb[c][c];
-        for (int r = c - 1; r >= 0; --r) {
-            double s = 0.0;
-            for (int p = r + 1; p <= c; ++p) s += Tb[r][p] * X[p][c];
-            X[r][c] = unit ? -s : -s / Tb[r][r];
-        }
+#pragma unroll
+        for (int r = 0; r < 16; ++r)
+            if (r >= c) X[(b0 + r) * TI_LD + b0 + c] = x[r];
     }
     __syncthreads();
-    TT *D = dinv + (int64_t)q * TH * TH;
-    for (int r = 0; r < TH; ++r) D[r + TH * c] = (TT)X[r][c];
+    // 16 -> 32: C A^-1 into the unused upper block of L, then -D^-1 (C A^-1)
+    {
+        const int b0 = tid < TI_NT / 2 ? 0 : 32, p = tid % (TI_NT / 2);
+        double *Lb = L + b0 * TI_LD + b0, *Xb = X + b0 * TI_LD + b0;
+        ti_product(Lb + 16, Lb + 16 * TI_LD, Xb, 16, 1.0, p, TI_NT / 2);
+        __syncthreads();
+        ti_product(Xb + 16 * TI_LD, Xb + 16 * TI_LD + 16, Lb + 16, 16, -1.0, p, TI_NT / 2);
+    }
+    __syncthreads();
+    // 32 -> 64
+    ti_product(L + 32, L + 32 * TI_LD, X, 32, 1.0, tid, TI_NT);
+    __syncthreads();
+    ti_product(X + 32 * TI_LD, X + 32 * TI_LD + 32, L + 32, 32, -1.0, tid, TI_NT);
+    __syncthreads();
+    TT *D = dinv + (int64_t)q * TH * TH;           // column-major
+    for (int idx = tid; idx < TH * TH; idx += TI_NT) {
+        const int c = idx / TH, r = idx % TH;
+        D[idx] = (TT)X[lower ? r * TI_LD + c : c * TI_LD + r];
+    }
 }
 
 // ------------------------------------------------------------------------
@@ -287,7 +336,7 @@ static int trtri_blocks(const TT *T, int64_t ldt, int64_t n, int h, char uplo, i
     const int64_t nb = (n + TH - 1) / TH;
     const int smem = 2 * TH * (TH + 1) * (int)sizeof(double);
     cudaFuncSetAttribute(k_trtri_blocks<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k_trtri_blocks<TT><<<(unsigned)nb, TH, smem, s>>>(T, ldt, n, uplo, unit, dinv);
+    k_trtri_blocks<TT><<<(unsigned)nb, TI_NT, smem, s>>>(T, ldt, n, uplo, unit, dinv);
     lnb_prof_count(1);
     return (int)cudaGetLastError();
 }
@@ -320,25 +369,29 @@ static int trsm_left(char uplo, char trans, int64_t n, int64_t nrhs, double alph
             return lnb_k_trsm_chain_f32(uplo, trans, n, nrhs, (const float *)T, ldt, (const float *)dinv, B, ldb,
                                         sync, st, wait_ns, s);
     }
-    TrsmArgs<TT> a;
-    a.T = T; a.ldt = ldt; a.dinv = dinv; a.B = B; a.ldb = ldb; a.n = n; a.nrhs = nrhs;
-    a.nb = (int)((n + TH - 1) / TH);
-    const bool lowerop = (uplo == 'L') == (trans == 'N');
-    a.fwd = lowerop ? 1 : 0;
-    a.tT = (trans == 'T') ? 1 : 0;
-    a.ticket = sync; a.cnt = sync + 4; a.ready = sync + 4 + a.nb;
-    a.st = st; a.wait_ns = wait_ns;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t items = 1 + (int64_t)a.nb * (a.nb - 1) / 2;
-    int64_t grid = (int64_t)sms * 4;
-    if (grid > items) grid = items;
-    const int smem = 3 * TH * TLD * (int)sizeof(double);
-    cudaFuncSetAttribute(k_trsm_dag<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k_trsm_dag<TT><<<(unsigned)grid, 128, smem, s>>>(a);
-    lnb_prof_count(1);
-    return (int)cudaGetLastError();
+    if constexpr (sizeof(TT) == 8) {
+        return (int)cudaErrorInvalidValue;         // k_trsm_tiles.cu takes these
+    } else {
+        TrsmArgs<TT> a;
+        a.T = T; a.ldt = ldt; a.dinv = dinv; a.B = B; a.ldb = ldb; a.n = n; a.nrhs = nrhs;
+        a.nb = (int)((n + TH - 1) / TH);
+        const bool lowerop = (uplo == 'L') == (trans == 'N');
+        a.fwd = lowerop ? 1 : 0;
+        a.tT = (trans == 'T') ? 1 : 0;
+        a.ticket = sync; a.cnt = sync + 4; a.ready = sync + 4 + a.nb;
+        a.st = st; a.wait_ns = wait_ns;
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const int64_t items = 1 + (int64_t)a.nb * (a.nb - 1) / 2;
+        int64_t grid = (int64_t)sms * 4;
+        if (grid > items) grid = items;
+        const int smem = 3 * TH * TLD * (int)sizeof(double);
+        cudaFuncSetAttribute(k_trsm_dag<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        k_trsm_dag<TT><<<(unsigned)grid, 128, smem, s>>>(a);
+        lnb_prof_count(1);
+        return (int)cudaGetLastError();
+    }
 }
 
 extern "C" int lnb_k_trtri_blocks_f64(const double *T, int64_t ldt, int64_t n, int h, char uplo, int unit,

@@ -69,6 +69,12 @@ int lnb_k_trtri_blocks_f64(const double *T, int64_t ldt, int64_t n, int h, char 
  * bounded by wait_ns of device time (st->timeout set on expiry).
  * sync: device scratch of lnb_trsm_sync_ints(n, h) ints (zeroed here). */
 int64_t lnb_trsm_sync_ints(int64_t n, int h);
+/* the same with more than 8 right-hand sides (k_trsm_tiles.cu): 64 x NW tiles of
+ * X, alpha folded in; sync: lnb_trsm_tiles_ints(nrhs) ints (zeroed here) */
+int64_t lnb_trsm_tiles_ints(int64_t nrhs);
+int lnb_k_trsm_tiles_f64(char uplo, char trans, int64_t n, int64_t nrhs, double alpha, const double *T, int64_t ldt,
+                         const double *dinv, double *B, int64_t ldb, int *sync, lnb_status_t *st, long long wait_ns,
+                         int sms, lnb_stream_t s);
 /* ticket0: first work item handed out (0; > 0 only in the wait self-test,
  * where skipping item 0 leaves a dependency that is never satisfied). */
 int lnb_k_trsm_left_f64(char uplo, char trans, int64_t n, int64_t nrhs, double alpha,

@@ -4,10 +4,10 @@
  * bblas_dltrsm (bblas_trsm.h:116-202) walks block rows issuing one TRSM task
  * per diagonal block and one GEMM task per off-diagonal block; spdsolv_main
  * (spdsolv_main.c:10-20) runs it twice, L Y = B then L^T X = Y.  Here each
- * solve is one persistent DAG-walking launch (k_trsv.cu) after one launch
- * that inverts the 64 x 64 diagonal blocks; the forward and the backward
- * solve share the inverses.  With many right-hand sides the solve is instead
- * a sequence of DMMA GEMMs over 64-row blocks (trsm_gemm).
+ * solve is one persistent DAG-walking launch (k_trsv_chain.cu, or
+ * k_trsm_tiles.cu with more than 8 right-hand sides) after one launch that
+ * inverts the 64 x 64 diagonal blocks; the forward and the backward solve share
+ * the inverses.
  */
 #include <stdlib.h>
 #include <string.h>
@@ -24,65 +24,16 @@
 
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-/* Two schedules for a solve: one persistent launch that walks the tile DAG,
- * or a sequence of DMMA GEMMs over 64-row blocks.  The DAG walk costs about
- * linearly in the right-hand sides; the GEMM sequence about 10 us per launch
- * plus full-rate tiles.  Measured on B200 (m = 1024 .. 16384), the GEMM
- * sequence wins from 128 - 256 columns on; auto switches at 192.  The GEMM
- * path needs at least TRSM_GEMM_MIN_NRHS columns (its workspace). */
-#define TRSM_GEMM_MIN_NRHS 32
-#define TRSM_GEMM_AUTO_NRHS 192
+/* Up to 8 right-hand sides take the chain walk (k_trsv_chain.cu), more the
+ * tile walk (k_trsm_tiles.cu). */
+#define TRSM_CHAIN_MAX_NRHS 8
 
 size_t lnb_trsm_f64_ws_bytes(int64_t n, int64_t nrhs)
 {
     const int64_t nb = ceil_div(n, TRSV_H);
+    const int64_t i1 = lnb_trsm_sync_ints(n, TRSV_H), i2 = lnb_trsm_tiles_ints(nrhs);
     return lnb_align256((size_t)nb * TRSV_H * TRSV_H * sizeof(double)) +
-           lnb_align256((size_t)lnb_trsm_sync_ints(n, TRSV_H) * sizeof(int)) +
-           (nrhs >= TRSM_GEMM_MIN_NRHS ? lnb_align256((size_t)TRSV_H * nrhs * sizeof(double)) : 0) + 512;
-}
-
-static int trsm_use_gemm(int64_t n, int64_t nrhs)
-{
-    static int mode = -2;
-    if (mode == -2) {
-        const char *e = getenv("LNB_TRSM_GEMM");    /* 0: always the DAG walk, 1: the GEMM path from 32 columns */
-        mode = e ? atoi(e) : -1;
-    }
-    if (nrhs < TRSM_GEMM_MIN_NRHS || mode == 0) return 0;
-    return mode == 1 || nrhs >= TRSM_GEMM_AUTO_NRHS;
-}
-
-/* op(T) X = alpha B by 64-row blocks in dependency order, the blocked solve of
- * bblas_dltrsm (bblas_trsm.h:119-160) with each TRSM task replaced by a
- * product with the inverted diagonal block:
- *     X_j = op(D_j) B_j                    (into tmp, then back into B_j)
- *     B_r = B_r - op(T)_{r,j} X_j          (every block row r still to come)
- * alpha enters through the first step: its diagonal product is scaled by
- * alpha and its update scales the rows still to come (beta = alpha), so
- * every later block already holds alpha B. */
-static int trsm_gemm(char uplo, char trans, int64_t n, int64_t nrhs, double alpha, const double *T, int64_t ldt,
-                     const double *dinv, double *B, int64_t ldb, double *tmp, cudaStream_t s)
-{
-    const int fwd = (uplo == 'L') == (trans == 'N');
-    const int64_t nb = ceil_div(n, TRSV_H);
-    for (int64_t q = 0; q < nb; ++q) {
-        const int64_t j = fwd ? q : nb - 1 - q;
-        const int64_t j0 = j * TRSV_H, jb = n - j0 < TRSV_H ? n - j0 : TRSV_H;
-        CK(lnb_k_gemm_tri_f64(trans, 'N', jb, nrhs, jb, q == 0 ? alpha : 1.0, dinv + j * TRSV_H * TRSV_H, TRSV_H,
-                              B + j0, ldb, 0.0, tmp, TRSV_H, 0, s), "diagonal block");
-        CK(cudaMemcpy2DAsync(B + j0, (size_t)ldb * 8, tmp, TRSV_H * 8, (size_t)jb * 8, nrhs, cudaMemcpyDeviceToDevice,
-                             s), "block back");
-        const int64_t r0 = fwd ? j0 + jb : 0, nr = fwd ? n - j0 - jb : j0;
-        if (nr <= 0) continue;
-        /* op(T)_{r,j}: stored at rows r, columns j (below the diagonal block
-         * for (L,N), above it for (U,N)); for trans 'T' it is the transpose of
-         * the block at rows j, columns r (left of the diagonal block for
-         * (L,T), right of it for (U,T)) */
-        const double *Ap = trans == 'N' ? T + r0 + j0 * ldt : T + j0 + r0 * ldt;
-        CK(lnb_k_gemm_tri_f64(trans, 'N', nr, nrhs, jb, -1.0, Ap, ldt, tmp, TRSV_H, q == 0 ? alpha : 1.0, B + r0, ldb,
-                              0, s), "update");
-    }
-    return 0;
+           lnb_align256((size_t)(i1 > i2 ? i1 : i2) * sizeof(int)) + 512;
 }
 
 /* op(T) X = alpha B with T triangular (uplo as stored), left side */
@@ -102,10 +53,12 @@ int lnb_trsm_f64_run(lnb_ctx *c, char uplo, char trans, char diag, int64_t n, in
         if (!dinv) return lnb_set_error(LNB_ENOMEM, "trsm workspace");
         CK(lnb_k_trtri_blocks_f64(dT, ldt, n, TRSV_H, uplo, diag == 'U', dinv, s), "trtri");
     }
-    if (trsm_use_gemm(n, nrhs)) {
-        double *tmp = (double *)lnb_arena_take(ar, (size_t)TRSV_H * nrhs * sizeof(double));
-        if (!tmp) return lnb_set_error(LNB_ENOMEM, "trsm workspace");
-        return trsm_gemm(uplo, trans, n, nrhs, alpha, dT, ldt, dinv, dB, ldb, tmp, s);
+    if (nrhs > TRSM_CHAIN_MAX_NRHS) {
+        int *sync = (int *)lnb_arena_take(ar, (size_t)lnb_trsm_tiles_ints(nrhs) * sizeof(int));
+        if (!sync) return lnb_set_error(LNB_ENOMEM, "trsm sync workspace");
+        CK(lnb_k_trsm_tiles_f64(uplo, trans, n, nrhs, alpha, dT, ldt, dinv, dB, ldb, sync, c->st, lnb_wait_ns(),
+                                c->sms, s), "trsm tiles");
+        return 0;
     }
     int *sync = (int *)lnb_arena_take(ar, (size_t)lnb_trsm_sync_ints(n, TRSV_H) * sizeof(int));
     if (!sync) return lnb_set_error(LNB_ENOMEM, "trsm sync workspace");
