@@ -52,7 +52,7 @@ struct BSmem {
     static constexpr size_t P = sizeof(TF) * BP * BLDP;              // panel, P[c][r] (factor phase)
     static constexpr size_t RS = sizeof(double) * BMAXR * BMAXN;      // r, z (solve phase, inside the panel)
     static constexpr size_t RED = sizeof(double) * (NT / 32) * BP * BMAXR;
-    static constexpr size_t SD = (size_t)bsd_bytes<TF>();               // staged block inverse (solve phase)
+    static constexpr size_t SD = 2 * (size_t)bsd_bytes<TF>();           // two staged block inverses (solve phase)
     static constexpr size_t PR = P > RS + RED + SD ? P : RS + RED + SD;
     static constexpr size_t LI = sizeof(TF) * BP * (BP + 1);         // block inverse, Li[p][j] = inv[j][p]
     static constexpr size_t RD = sizeof(TF) * BP;                     // 1 / diagonal
@@ -119,8 +119,9 @@ __device__ double bresidual(const double *A, int n, int nr, const double *B, con
     return worst;
 }
 
+// two FP32 systems of 256 threads share an SM: 128 registers per thread
 template <typename TF, int NT>
-__global__ void __launch_bounds__(NT) k_batched_posv(BatchArgs a)
+__global__ void __launch_bounds__(NT, sizeof(TF) == 4 && NT == 256 ? 2 : 1) k_batched_posv(BatchArgs a)
 {
     using SM = BSmem<TF, NT>;
     extern __shared__ __align__(16) unsigned char smb[];
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(NT) k_batched_posv(BatchArgs a)
             const double tol = a.tol_eps * n;
             const int maxit = (sizeof(TF) == 8) ? 1 : a.max_iter;
             for (it = 1; it <= maxit; ++it) {
-                bsolve<TF, NT>(F, ldF, Dv, n, nr, rs, red, sD);       // r <- M^-1 r
+                bsolve<TF, NT>(F, ldF, Dv, n, nr, rs, sD);       // r <- M^-1 r
                 for (int t = tid; t < n * nr; t += NT) {
                     const int i = t % n, q = t / n;
                     xs[q * BMAXN + i] += rs[q * BMAXN + i];
