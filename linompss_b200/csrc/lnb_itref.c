@@ -6,8 +6,9 @@
  * tmp = A p, alpha2 = <tmp,p>, x += (alpha1/alpha2) p, r -= (alpha1/alpha2)
  * tmp, alpha1 = <r,r>, then the direction update as the reference executes
  * it (p = 2 r, see k_blas1.cu), and the relative test ||r||/||b|| <= tol.
- * The scalars never leave the device except the one norm per step that the
- * stopping test needs (the reference's taskwait, itref.c:830).
+ * Up to n = 12288 a solve is one launch, the stopping test (the reference's
+ * taskwait, itref.c:830) on the device; above, the scalars never leave the device
+ * except the one norm per step that the test needs.
  *
  * ompss_ditref restates the outer loop of itref.c:999-1101.
  */
@@ -28,24 +29,32 @@ typedef struct {
     double *r, *p, *tmp;       /* n each */
     double *scal;              /* [0]=alpha1 [1]=alpha2 [2]=<b,b> [3]=spare */
     double *part, *dpart;
+    int *sync;                 /* the one-launch form's counters */
 } cg_ws;
 
-static size_t cg_ws_bytes(int64_t n)
+static int64_t cg_part_doubles(int64_t n, int sms)
 {
-    return 3 * lnb_align256((size_t)n * 8) + lnb_align256(8 * 8) +
-           lnb_align256((size_t)lnb_gemv_part_doubles(n, n) * 8) +
+    const int64_t g = lnb_gemv_part_doubles(n, n), d = n <= lnb_dcg_max_n() ? lnb_dcg_part_doubles(n, sms) : 0;
+    return g > d ? g : d;
+}
+
+static size_t cg_ws_bytes(int64_t n, int sms)
+{
+    return 3 * lnb_align256((size_t)n * 8) + lnb_align256(8 * 8) + lnb_align256(64 * sizeof(int)) +
+           lnb_align256((size_t)cg_part_doubles(n, sms) * 8) +
            lnb_align256((size_t)lnb_dot_part_doubles(n) * 8) + 2048;
 }
 
-static int cg_ws_take(lnb_arena *ar, int64_t n, cg_ws *w)
+static int cg_ws_take(lnb_arena *ar, int64_t n, int sms, cg_ws *w)
 {
     w->r = lnb_arena_take(ar, (size_t)n * 8);
     w->p = lnb_arena_take(ar, (size_t)n * 8);
     w->tmp = lnb_arena_take(ar, (size_t)n * 8);
     w->scal = lnb_arena_take(ar, 8 * 8);
-    w->part = lnb_arena_take(ar, (size_t)lnb_gemv_part_doubles(n, n) * 8);
+    w->sync = lnb_arena_take(ar, 64 * sizeof(int));
+    w->part = lnb_arena_take(ar, (size_t)cg_part_doubles(n, sms) * 8);
     w->dpart = lnb_arena_take(ar, (size_t)lnb_dot_part_doubles(n) * 8);
-    return (w->r && w->p && w->tmp && w->scal && w->part && w->dpart) ? 0
+    return (w->r && w->p && w->tmp && w->scal && w->sync && w->part && w->dpart) ? 0
                                                                        : lnb_set_error(LNB_ENOMEM, "cg workspace");
 }
 
@@ -54,6 +63,16 @@ static int cg_ws_take(lnb_arena *ar, int64_t n, cg_ws *w)
 static int dcg_dev(lnb_ctx *c, int64_t n, const double *dA, int64_t lda, const double *db, double *dx,
                    double tol, int steps, int mode, cg_ws *w, cudaStream_t s)
 {
+    if (!mode && n <= lnb_dcg_max_n()) {
+        /* the whole solve in one launch */
+        int h2[2];
+        CK(cudaMemsetAsync(c->st, 0, sizeof(lnb_status_t), s), "status reset");
+        CK(lnb_k_dcg_f64(n, dA, lda, db, dx, tol, steps, w->part, w->sync, c->st, lnb_wait_ns(), c->sms, s), "dcg");
+        CK(cudaMemcpyAsync(h2, w->sync + 32, sizeof h2, cudaMemcpyDeviceToHost, s), "read");
+        const int e = lnb_status_read(c, s);
+        if (e < 0) return e < -1 ? e : LNB_ECUDA;
+        return h2[1] ? -1 : h2[0];
+    }
     double *a1 = w->scal, *a2 = w->scal + 1, *bb = w->scal + 2;
     double h[2];
     CK(lnb_k_dot_f64(n, db, db, bb, w->dpart, s), "dot");
@@ -100,14 +119,14 @@ int ompss_dcg(int n, int bm, const double *A, int lda, const double *b, double *
     lnb_ctx *c = lnb_ctx_get();
     if (!c) return LNB_ENODEV;
     const int64_t ldd = (n + 7) & ~7;
-    void *ws = lnb_ws(c, lnb_align256((size_t)ldd * n * 8) + 2 * lnb_align256((size_t)n * 8) + cg_ws_bytes(n));
+    void *ws = lnb_ws(c, lnb_align256((size_t)ldd * n * 8) + 2 * lnb_align256((size_t)n * 8) + cg_ws_bytes(n, c->sms));
     if (!ws) return LNB_ENOMEM;
     lnb_arena ar = {(char *)ws, 0, c->ws_size};
     double *dA = lnb_arena_take(&ar, (size_t)ldd * n * 8);
     double *db = lnb_arena_take(&ar, (size_t)n * 8), *dx = lnb_arena_take(&ar, (size_t)n * 8);
     cg_ws w;
     int e;
-    if ((e = cg_ws_take(&ar, n, &w))) return e;
+    if ((e = cg_ws_take(&ar, n, c->sms, &w))) return e;
     cudaStream_t s = c->main;
     if ((e = copy_in_matrix(dA, ldd, A, lda, n, s))) return e;
     CK(cudaMemcpyAsync(db, b, (size_t)n * 8, cudaMemcpyHostToDevice, s), "b in");
@@ -129,7 +148,7 @@ int ompss_ditref(int n, int bm, const double *A, int lda, const double *b, doubl
     lnb_ctx *c = lnb_ctx_get();
     if (!c) return LNB_ENODEV;
     const int64_t ldd = (n + 7) & ~7;
-    void *ws = lnb_ws(c, lnb_align256((size_t)ldd * n * 8) + 8 * lnb_align256((size_t)n * 8) + cg_ws_bytes(n) + 512);
+    void *ws = lnb_ws(c, lnb_align256((size_t)ldd * n * 8) + 8 * lnb_align256((size_t)n * 8) + cg_ws_bytes(n, c->sms) + 512);
     if (!ws) return LNB_ENOMEM;
     lnb_arena ar = {(char *)ws, 0, c->ws_size};
     double *dA = lnb_arena_take(&ar, (size_t)ldd * n * 8);
@@ -143,7 +162,7 @@ int ompss_ditref(int n, int bm, const double *A, int lda, const double *b, doubl
     double *r2 = lnb_arena_take(&ar, 2 * 8);
     cg_ws w;
     int e;
-    if ((e = cg_ws_take(&ar, n, &w))) return e;
+    if ((e = cg_ws_take(&ar, n, c->sms, &w))) return e;
     cudaStream_t s = c->main;
     if ((e = copy_in_matrix(dA, ldd, A, lda, n, s))) return e;
     CK(cudaMemcpyAsync(rhs, b, (size_t)n * 8, cudaMemcpyHostToDevice, s), "b in");

@@ -154,6 +154,12 @@ int lnb_k_axpy_scaled_f64(int64_t n, int64_t nrhs, const double *sc, const doubl
 void lnb_prof_count(int kernels);
 
 /* ---- FP64 vector kernels (k_blas1.cu); reductions are deterministic ------- */
+/* dcg_pure (the reference's recurrence) as one cooperative launch, n <= lnb_dcg_max_n(): x the start vector on entry,
+ * the iterate on exit; part: lnb_dcg_part_doubles(n, sms); sync: 64 ints, [32] steps done and [33] converged on return */
+int64_t lnb_dcg_max_n(void);
+int64_t lnb_dcg_part_doubles(int64_t n, int sms);
+int lnb_k_dcg_f64(int64_t n, const double *A, int64_t lda, const double *b, double *x, double tol, int steps,
+                  double *part, int *sync, lnb_status_t *st, long long wait_ns, int sms, lnb_stream_t s);
 int64_t lnb_gemv_part_doubles(int64_t m, int64_t n);
 int64_t lnb_dot_part_doubles(int64_t n);
 /* y = alpha A x + beta yin (A m x n).  If dot_out: *dot_out = <y, w>.
