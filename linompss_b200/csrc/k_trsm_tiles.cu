@@ -1,5 +1,5 @@
-// k_trsm_tiles.cu -- op(T) X = alpha B in FP64 with more than a few right-hand
-// sides, as one persistent launch that walks the tile DAG.
+// k_trsm_tiles.cu -- op(T) X = alpha B in FP64 as one persistent launch that walks
+// the tile DAG.
 //
 // Semantics of bblas_dltrsm (bblas_trsm.h:116-202): block rows in dependency
 // order, a TRSM task on each diagonal block and a GEMM task per off-diagonal
@@ -18,11 +18,13 @@
 //     waits only on smaller tickets; every wait is bounded and reports in the
 //     status word.
 //   * Bound by the DMMA rate when block rows x strips fill the SMs, by the chain
-//     of nb dependent tiles otherwise: a narrower strip shortens the chain's link
-//     (NW = 64, 32, 16: 8.9, 6, 4.9 us) at the price of rereading T.  n = 1500 with
-//     1500 columns takes 0.21 ms (0.96 as two GEMM launches per block row), n =
-//     16384 with 64 1.7 ms (3.85 as a walk of 64 x 64 updates with atomics); with
-//     n = 8192 and 4096 columns it runs at 27.6 TF/s.
+//     of nb dependent tiles otherwise: 3.5 us per link with NW = 16 (flag seen 0.3,
+//     X in 0.4, four chunks 1.2, right-hand side and inverse 0.4, stores and flag
+//     1.1); wider strips lengthen the link and reread T less.  n = 8192 with one
+//     right-hand side takes 0.45 ms per solve (0.64 as a substitution chain in one
+//     CTA with two blocks of band), n = 1500 with 1500 columns 0.21 ms (0.96 as two
+//     GEMM launches per block row), n = 16384 with 64 1.4 ms (3.85 as a walk of
+//     64 x 64 updates with atomics); n = 8192 with 4096 columns runs at 27.6 TF/s.
 #include "common.cuh"
 #include "tc_sm100.cuh"
 
@@ -52,6 +54,7 @@ struct Args {
     int nb, ns, fwd;
     int64_t ntasks;
     int *ticket, *prog;             // prog[s]: tiles of strip s that are final
+    int ticket0;                    // first ticket handed out (0; 1 only in the wait self-test)
     lnb_status_t *st;
     long long wait_ns;
 };
@@ -113,7 +116,8 @@ LNB_DEV void cp8(uint32_t d, const double *g, int bytes)
 }
 
 // NC columns of 64 contiguous elements: dst[c * LDC + r] = X[r + c ld], zero where
-// r >= nr or c >= nc; by the producer warp
+// r >= nr or c >= nc; by the producer warp.  Pointers step from column to column:
+// the warp issues alone, and its address arithmetic is the chunk's latency.
 template <int NC>
 LNB_DEV void load64(double *dst, const double *X, int64_t ld, int nr, int nc, bool vec, int lane)
 {
@@ -121,16 +125,24 @@ LNB_DEV void load64(double *dst, const double *X, int64_t ld, int nr, int nc, bo
         const int r = 2 * lane, bytes = r + 1 < nr ? 16 : r < nr ? 8 : 0;
         uint32_t d = smem_u32(dst + r);
         const double *g = X + (bytes ? r : 0);
-#pragma unroll 8
-        for (int c = 0; c < NC; ++c, d += LDC * 8) cp16(d, c < nc ? g + c * ld : X, c < nc ? bytes : 0);
+        if (nc >= NC) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c, g += ld) cp16(d + c * (LDC * 8), g, bytes);
+        } else {
+#pragma unroll 1
+            for (int c = 0; c < NC; ++c, d += LDC * 8) cp16(d, c < nc ? g + c * ld : X, c < nc ? bytes : 0);
+        }
     } else {
         const int b0 = lane < nr ? 8 : 0, b1 = lane + 32 < nr ? 8 : 0;
         uint32_t d = smem_u32(dst + lane);
         const double *g0 = X + (b0 ? lane : 0), *g1 = X + (b1 ? lane + 32 : 0);
-#pragma unroll 8
+#pragma unroll 4
         for (int c = 0; c < NC; ++c, d += LDC * 8) {
-            cp8(d, c < nc ? g0 + c * ld : X, c < nc ? b0 : 0);
-            cp8(d + 256, c < nc ? g1 + c * ld : X, c < nc ? b1 : 0);
+            const bool in = c < nc;
+            cp8(d, in ? g0 : X, in ? b0 : 0);
+            cp8(d + 256, in ? g1 : X, in ? b1 : 0);
+            g0 += ld;
+            g1 += ld;
         }
     }
 }
@@ -142,16 +154,24 @@ LNB_DEV void load16(double *dst, const double *X, int64_t ld, int nr, int nc, bo
         const int r = 2 * (lane & 7), bytes = r + 1 < nr ? 16 : r < nr ? 8 : 0;
         int c = lane >> 3;
         uint32_t d = smem_u32(dst + c * LDR + r);
-        const double *g = X + (bytes ? r : 0);
-#pragma unroll 8
-        for (int it = 0; it < NC / 4; ++it, c += 4, d += 4 * LDR * 8) cp16(d, c < nc ? g + c * ld : X, c < nc ? bytes : 0);
+        const double *g = X + (bytes ? r : 0) + c * ld;
+        const int64_t step = 4 * ld;
+        if (nc >= NC) {
+#pragma unroll
+            for (int it = 0; it < NC / 4; ++it, g += step) cp16(d + it * (4 * LDR * 8), g, bytes);
+        } else {
+#pragma unroll 1
+            for (int it = 0; it < NC / 4; ++it, c += 4, d += 4 * LDR * 8, g += step)
+                cp16(d, c < nc ? g : X, c < nc ? bytes : 0);
+        }
     } else {
         const int r = lane & 15, bytes = r < nr ? 8 : 0;
         int c = lane >> 4;
         uint32_t d = smem_u32(dst + c * LDR + r);
-        const double *g = X + (bytes ? r : 0);
-#pragma unroll 8
-        for (int it = 0; it < NC / 2; ++it, c += 2, d += 2 * LDR * 8) cp8(d, c < nc ? g + c * ld : X, c < nc ? bytes : 0);
+        const double *g = X + (bytes ? r : 0) + c * ld;
+        const int64_t step = 2 * ld;
+#pragma unroll 4
+        for (int it = 0; it < NC / 2; ++it, c += 2, d += 2 * LDR * 8, g += step) cp8(d, c < nc ? g : X, c < nc ? bytes : 0);
     }
 }
 
@@ -173,23 +193,34 @@ LNB_DEV bool produce(const Args &a, int v, int s, double *sm, Shared &sh, int &q
     arrive_copied(&sh.dfull);
     int known = 0;
     bool ok = true;
-    const int nch = v * (TS / BK);
-    for (int c = 0; c < nch; ++c, ++q) {
-        const int st = q % C::ST;
-        if (q >= C::ST && !bar_wait(&sh.empty[st], ((q / C::ST) - 1) & 1, 4 * a.wait_ns, sh)) ok = false;
-        if (!__all_sync(0xffffffffu, ok)) {
-            ok = false;
-            break;
-        }
-        double *as = sm + st * C::STAGE, *bs = as + ACH;
-        const int u = c / (TS / BK);
-        const int64_t oj = (int64_t)(a.fwd ? u : a.nb - 1 - u) * TS, k0 = oj + (c % (TS / BK)) * BK;
-        const int kn = (int)(a.n - k0 < 0 ? 0 : a.n - k0 < BK ? a.n - k0 : BK);
-        // op(T)(m, k) = T[oi + m + (k0 + k) ldt], or T[k0 + k + (oi + m) ldt]
-        const int64_t kc = kn > 0 ? k0 : 0;
-        if (!TR) load64<BK>(as, a.T + oi + kc * a.ldt, a.ldt, rows, kn, vt, lane);
-        else load16<TS>(as, a.T + kc + oi * a.ldt, a.ldt, kn, rows, vt, lane);
+    constexpr int CPT = TS / BK;                     // chunks per tile
+    for (int u = 0; u < v && ok; ++u) {
+        const int64_t oj = (int64_t)(a.fwd ? u : a.nb - 1 - u) * TS;     // block u in solve order
+        const int kt = blk_len(a, oj);
+        // op(T)(m, k) = T[oi + m + (oj + k) ldt], or T[oj + k + (oi + m) ldt]
+        const double *Tu = a.T + (TR ? oj + oi * a.ldt : oi + oj * a.ldt);
+        const double *Bu = a.B + oj + c0 * a.ldb;
+        auto load_t = [&](int c) {                   // chunk c of the tile, into the slot of chunk q + c
+            const int qc = q + c, st = qc % C::ST;
+            if (qc >= C::ST && !bar_wait(&sh.empty[st], ((qc / C::ST) - 1) & 1, 4 * a.wait_ns, sh)) ok = false;
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) return;
+            const int kn = kt - c * BK < 0 ? 0 : kt - c * BK < BK ? kt - c * BK : BK;
+            double *as = sm + st * C::STAGE;
+            if (!TR) load64<BK>(as, kn ? Tu + c * BK * a.ldt : a.T, a.ldt, rows, kn, vt, lane);
+            else load16<TS>(as, kn ? Tu + c * BK : a.T, a.ldt, kn, rows, vt, lane);
+        };
+        auto load_b = [&](int c) {
+            const int st = (q + c) % C::ST;
+            const int kn = kt - c * BK < 0 ? 0 : kt - c * BK < BK ? kt - c * BK : BK;
+            load16<NW>(sm + st * C::STAGE + ACH, kn ? Bu + c * BK : a.B, a.ldb, kn, cols, vb, lane);
+            arrive_copied(&sh.full[st]);
+        };
+        int ahead = 0;                               // chunks whose part of T goes out before the wait
         if (u >= known) {
+            constexpr int AH = C::ST < CPT ? C::ST : CPT;
+            for (; ahead < AH && ok; ++ahead) load_t(ahead);
+            if (!ok) break;
             if (lane == 0) known = wait_prog(a.prog + s, u + 1, a);
             known = __shfl_sync(0xffffffffu, known, 0);
             if (known < 0) {
@@ -197,8 +228,11 @@ LNB_DEV bool produce(const Args &a, int v, int s, double *sm, Shared &sh, int &q
                 break;
             }
         }
-        load16<NW>(bs, a.B + kc + c0 * a.ldb, a.ldb, kn, cols, vb, lane);
-        arrive_copied(&sh.full[st]);
+        for (int c = 0; c < CPT && ok; ++c) {
+            if (c >= ahead) load_t(c);
+            if (ok) load_b(c);
+        }
+        q += CPT;
     }
     if (!ok) {
         if (lane == 0) {
@@ -336,7 +370,7 @@ __global__ void __launch_bounds__(NTHR, 2) k_trsm_tiles(Args a)
     for (;;) {
         __syncthreads();
         if (*(volatile int *)&sh.abort) break;       // the same for every thread: set before the barrier
-        if (threadIdx.x == 0) sh.task = atomicAdd(a.ticket, 1);
+        if (threadIdx.x == 0) sh.task = atomicAdd(a.ticket, 1) + a.ticket0;
         __syncthreads();
         const int tk = sh.task;
         if (tk >= a.ntasks) break;
@@ -368,7 +402,7 @@ extern "C" int64_t lnb_trsm_tiles_ints(int64_t nrhs) { return 32 + (nrhs + 15) /
 // inverses of T's diagonal blocks; sync: lnb_trsm_tiles_ints(nrhs) ints (zeroed here)
 extern "C" int lnb_k_trsm_tiles_f64(char uplo, char trans, int64_t n, int64_t nrhs, double alpha, const double *T,
                                     int64_t ldt, const double *dinv, double *B, int64_t ldb, int *sync,
-                                    lnb_status_t *st, long long wait_ns, int sms, lnb_stream_t s)
+                                    lnb_status_t *st, long long wait_ns, int sms, int ticket0, lnb_stream_t s)
 {
     using namespace lnb::tiles;
     if (n <= 0 || nrhs <= 0) return 0;
@@ -384,7 +418,7 @@ extern "C" int lnb_k_trsm_tiles_f64(char uplo, char trans, int64_t n, int64_t nr
     a.nb = (int)nb; a.ns = (int)((nrhs + nw - 1) / nw); a.fwd = (uplo == 'L') == (trans == 'N');
     a.ntasks = nb * a.ns;
     if (a.ntasks > INT32_MAX - 1024) return (int)cudaErrorInvalidValue;
-    a.ticket = sync; a.prog = sync + 32; a.st = st; a.wait_ns = wait_ns;
+    a.ticket = sync; a.ticket0 = ticket0; a.prog = sync + 32; a.st = st; a.wait_ns = wait_ns;
     const cudaError_t e = cudaMemsetAsync(sync, 0, (size_t)lnb_trsm_tiles_ints(nrhs) * sizeof(int), (cudaStream_t)s);
     if (e != cudaSuccess) return (int)e;
     const bool tr = trans == 'T';

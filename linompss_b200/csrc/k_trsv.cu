@@ -341,9 +341,9 @@ static int trtri_blocks(const TT *T, int64_t ldt, int64_t n, int h, char uplo, i
     return (int)cudaGetLastError();
 }
 
-template <typename TT>
-static int trsm_left(char uplo, char trans, int64_t n, int64_t nrhs, double alpha, const TT *T, int64_t ldt,
-                     const TT *dinv, int h, double *B, int64_t ldb, int *sync, lnb_status_t *st,
+// FP32 T
+static int trsm_left(char uplo, char trans, int64_t n, int64_t nrhs, double alpha, const float *T, int64_t ldt,
+                     const float *dinv, int h, double *B, int64_t ldb, int *sync, lnb_status_t *st,
                      long long wait_ns, int ticket0, lnb_stream_t s)
 {
     if (h != TH) return (int)cudaErrorInvalidValue;
@@ -361,37 +361,27 @@ static int trsm_left(char uplo, char trans, int64_t n, int64_t nrhs, double alph
         e = cudaMemsetAsync(sync, ticket0 & 0xff, 1, s);  // ticket starts past item 0
         if (e != cudaSuccess) return (int)e;
     }
-    if (nrhs <= 8) {
-        if constexpr (sizeof(TT) == 8)
-            return lnb_k_trsm_chain_f64(uplo, trans, n, nrhs, (const double *)T, ldt, (const double *)dinv, B, ldb,
-                                        sync, st, wait_ns, s);
-        else
-            return lnb_k_trsm_chain_f32(uplo, trans, n, nrhs, (const float *)T, ldt, (const float *)dinv, B, ldb,
-                                        sync, st, wait_ns, s);
-    }
-    if constexpr (sizeof(TT) == 8) {
-        return (int)cudaErrorInvalidValue;         // k_trsm_tiles.cu takes these
-    } else {
-        TrsmArgs<TT> a;
-        a.T = T; a.ldt = ldt; a.dinv = dinv; a.B = B; a.ldb = ldb; a.n = n; a.nrhs = nrhs;
-        a.nb = (int)((n + TH - 1) / TH);
-        const bool lowerop = (uplo == 'L') == (trans == 'N');
-        a.fwd = lowerop ? 1 : 0;
-        a.tT = (trans == 'T') ? 1 : 0;
-        a.ticket = sync; a.cnt = sync + 4; a.ready = sync + 4 + a.nb;
-        a.st = st; a.wait_ns = wait_ns;
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int64_t items = 1 + (int64_t)a.nb * (a.nb - 1) / 2;
-        int64_t grid = (int64_t)sms * 4;
-        if (grid > items) grid = items;
-        const int smem = 3 * TH * TLD * (int)sizeof(double);
-        cudaFuncSetAttribute(k_trsm_dag<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        k_trsm_dag<TT><<<(unsigned)grid, 128, smem, s>>>(a);
-        lnb_prof_count(1);
-        return (int)cudaGetLastError();
-    }
+    if (nrhs <= 8)
+        return lnb_k_trsm_chain_f32(uplo, trans, n, nrhs, T, ldt, dinv, B, ldb, sync, st, wait_ns, s);
+    TrsmArgs<float> a;
+    a.T = T; a.ldt = ldt; a.dinv = dinv; a.B = B; a.ldb = ldb; a.n = n; a.nrhs = nrhs;
+    a.nb = (int)((n + TH - 1) / TH);
+    const bool lowerop = (uplo == 'L') == (trans == 'N');
+    a.fwd = lowerop ? 1 : 0;
+    a.tT = (trans == 'T') ? 1 : 0;
+    a.ticket = sync; a.cnt = sync + 4; a.ready = sync + 4 + a.nb;
+    a.st = st; a.wait_ns = wait_ns;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t items = 1 + (int64_t)a.nb * (a.nb - 1) / 2;
+    int64_t grid = (int64_t)sms * 4;
+    if (grid > items) grid = items;
+    const int smem = 3 * TH * TLD * (int)sizeof(double);
+    cudaFuncSetAttribute(k_trsm_dag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    k_trsm_dag<float><<<(unsigned)grid, 128, smem, s>>>(a);
+    lnb_prof_count(1);
+    return (int)cudaGetLastError();
 }
 
 extern "C" int lnb_k_trtri_blocks_f64(const double *T, int64_t ldt, int64_t n, int h, char uplo, int unit,
@@ -404,15 +394,9 @@ extern "C" int lnb_k_trtri_blocks_f32(const float *T, int64_t ldt, int64_t n, in
 {
     return trtri_blocks<float>(T, ldt, n, h, uplo, unit, dinv, s);
 }
-extern "C" int lnb_k_trsm_left_f64(char uplo, char trans, int64_t n, int64_t nrhs, double alpha, const double *T,
-                                   int64_t ldt, const double *dinv, int h, double *B, int64_t ldb, int *sync,
-                                   lnb_status_t *st, long long wait_ns, int ticket0, lnb_stream_t s)
-{
-    return trsm_left<double>(uplo, trans, n, nrhs, alpha, T, ldt, dinv, h, B, ldb, sync, st, wait_ns, ticket0, s);
-}
 extern "C" int lnb_k_trsm_left_f32(char uplo, char trans, int64_t n, int64_t nrhs, double alpha, const float *T,
                                    int64_t ldt, const float *dinv, int h, double *B, int64_t ldb, int *sync,
                                    lnb_status_t *st, long long wait_ns, int ticket0, lnb_stream_t s)
 {
-    return trsm_left<float>(uplo, trans, n, nrhs, alpha, T, ldt, dinv, h, B, ldb, sync, st, wait_ns, ticket0, s);
+    return trsm_left(uplo, trans, n, nrhs, alpha, T, ldt, dinv, h, B, ldb, sync, st, wait_ns, ticket0, s);
 }

@@ -1,5 +1,6 @@
 // k_trsv_chain.cu -- blocked triangular solves with few right-hand sides
-// (nrhs <= 8): op(T) X = B, T triangular, FP64 arithmetic on FP64 or FP32 T.
+// (nrhs <= 8): op(T) X = B, T triangular, FP64 arithmetic on an FP32 T (FP64 T:
+// k_trsm_tiles.cu).
 //
 // Semantics of bblas_dltrsm (bblas_trsm.h:116-202) and of the two solves of
 // dspdsolv_main (spdsolv_main.c:15,17), as k_trsv.cu.  With one or a few
@@ -47,17 +48,14 @@ constexpr int PF = 4;               // L2 prefetch distance of the chain, in ste
 // band width W handled by the chain CTA, worker chunk CW (tiles per item)
 template <typename TT> struct Cfg;
 template <> struct Cfg<float> { static constexpr int W = 4, CW = 4; };
-template <> struct Cfg<double> { static constexpr int W = 2, CW = 2; };
 
 // Padded leading dimension of a staged 64 x 64 tile S[col * LD + row].
 // TR (op = transpose) reads rows of S with 16-byte vectors, 2 columns per
 // 8-lane phase: LD == 16 words mod 32.  !TR reads 4 columns x 8 rows per
-// phase (scalar): LD == 8 floats mod 32, or 4 doubles mod 16.
+// phase (scalar): LD == 8 floats mod 32.
 template <typename TT, bool TR> struct Ld;
 template <> struct Ld<float, true> { static constexpr int v = 80; };
 template <> struct Ld<float, false> { static constexpr int v = 72; };
-template <> struct Ld<double, true> { static constexpr int v = 72; };
-template <> struct Ld<double, false> { static constexpr int v = 68; };
 
 template <typename TT>
 struct Args {
@@ -320,7 +318,7 @@ struct ChainBars {
 // the s-th step (s >= 1) stages its band tiles into buffer s & 1: the phase of
 // tfull[s & 1] it completes
 LNB_DEV uint32_t tile_phase(int s) { return (uint32_t)(((s & 1) ? (s - 1) >> 1 : (s - 2) >> 1) & 1); }
-static_assert(Cfg<float>::W * 64 <= NCOMP && Cfg<double>::W * 64 <= NCOMP, "one tile column per compute thread");
+static_assert(Cfg<float>::W * 64 <= NCOMP, "one tile column per compute thread");
 
 // wait for copies this CTA issued before it leaves: bounded by budget_ns, and
 // unlike mbar_wait not cut short by an abort or a recorded timeout
@@ -797,13 +795,6 @@ int trsm_chain(char uplo, char trans, int64_t n, int64_t nrhs, const TT *T, int6
 }  // namespace lnb
 
 // sync must hold lnb_trsm_sync_ints(n, 64) zeroed ints (ticket first).
-extern "C" int lnb_k_trsm_chain_f64(char uplo, char trans, int64_t n, int64_t nrhs, const double *T, int64_t ldt,
-                                    const double *dinv, double *B, int64_t ldb, int *sync, lnb_status_t *st,
-                                    long long wait_ns, lnb_stream_t s)
-{
-    if (nrhs > 8) return (int)cudaErrorInvalidValue;
-    return lnb::chain::trsm_chain<double>(uplo, trans, n, nrhs, T, ldt, dinv, B, ldb, sync, st, wait_ns, s);
-}
 extern "C" int lnb_k_trsm_chain_f32(char uplo, char trans, int64_t n, int64_t nrhs, const float *T, int64_t ldt,
                                     const float *dinv, double *B, int64_t ldb, int *sync, lnb_status_t *st,
                                     long long wait_ns, lnb_stream_t s)

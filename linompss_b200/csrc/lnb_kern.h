@@ -67,27 +67,20 @@ int lnb_k_trtri_blocks_f64(const double *T, int64_t ldt, int64_t n, int h, char 
  * inverses from lnb_k_trtri_blocks_f64.  uplo/trans describe T as stored.
  * One persistent launch walks the solve's tile DAG; every dependency wait is
  * bounded by wait_ns of device time (st->timeout set on expiry).
- * sync: device scratch of lnb_trsm_sync_ints(n, h) ints (zeroed here). */
-int64_t lnb_trsm_sync_ints(int64_t n, int h);
-/* the same with more than 8 right-hand sides (k_trsm_tiles.cu): 64 x NW tiles of
- * X, alpha folded in; sync: lnb_trsm_tiles_ints(nrhs) ints (zeroed here) */
+ * FP64 T (k_trsm_tiles.cu): 64 x NW tiles of X, alpha folded in; sync:
+ * lnb_trsm_tiles_ints(nrhs) ints of device scratch (zeroed here).  ticket0:
+ * first task handed out (0; > 0 only in the wait self-test, where skipping
+ * task 0 leaves a dependency that is never satisfied). */
 int64_t lnb_trsm_tiles_ints(int64_t nrhs);
 int lnb_k_trsm_tiles_f64(char uplo, char trans, int64_t n, int64_t nrhs, double alpha, const double *T, int64_t ldt,
                          const double *dinv, double *B, int64_t ldb, int *sync, lnb_status_t *st, long long wait_ns,
-                         int sms, lnb_stream_t s);
-/* ticket0: first work item handed out (0; > 0 only in the wait self-test,
- * where skipping item 0 leaves a dependency that is never satisfied). */
-int lnb_k_trsm_left_f64(char uplo, char trans, int64_t n, int64_t nrhs, double alpha,
-                        const double *T, int64_t ldt, const double *dinv, int h, double *B,
-                        int64_t ldb, int *sync, lnb_status_t *st, long long wait_ns,
-                        int ticket0, lnb_stream_t s);
+                         int sms, int ticket0, lnb_stream_t s);
 
-/* Few right-hand sides (nrhs <= 8): the same solve as one launch built
- * around the diagonal chain (k_trsv_chain.cu).  sync as above, zeroed by the
- * caller; alpha already applied. */
-int lnb_k_trsm_chain_f64(char uplo, char trans, int64_t n, int64_t nrhs, const double *T, int64_t ldt,
-                         const double *dinv, double *B, int64_t ldb, int *sync, lnb_status_t *st,
-                         long long wait_ns, lnb_stream_t s);
+/* FP32 T: scratch of lnb_k_trsm_left_f32 (ints) */
+int64_t lnb_trsm_sync_ints(int64_t n, int h);
+/* FP32 T and few right-hand sides (nrhs <= 8): one launch built around the
+ * diagonal chain (k_trsv_chain.cu).  sync zeroed by the caller; alpha already
+ * applied. */
 int lnb_k_trsm_chain_f32(char uplo, char trans, int64_t n, int64_t nrhs, const float *T, int64_t ldt,
                          const float *dinv, double *B, int64_t ldb, int *sync, lnb_status_t *st,
                          long long wait_ns, lnb_stream_t s);

@@ -4,10 +4,9 @@
  * bblas_dltrsm (bblas_trsm.h:116-202) walks block rows issuing one TRSM task
  * per diagonal block and one GEMM task per off-diagonal block; spdsolv_main
  * (spdsolv_main.c:10-20) runs it twice, L Y = B then L^T X = Y.  Here each
- * solve is one persistent DAG-walking launch (k_trsv_chain.cu, or
- * k_trsm_tiles.cu with more than 8 right-hand sides) after one launch that
- * inverts the 64 x 64 diagonal blocks; the forward and the backward solve share
- * the inverses.
+ * solve is one persistent DAG-walking launch (k_trsm_tiles.cu) after one launch
+ * that inverts the 64 x 64 diagonal blocks; the forward and the backward solve
+ * share the inverses.
  */
 #include <stdlib.h>
 #include <string.h>
@@ -24,16 +23,11 @@
 
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-/* Up to 8 right-hand sides take the chain walk (k_trsv_chain.cu), more the
- * tile walk (k_trsm_tiles.cu). */
-#define TRSM_CHAIN_MAX_NRHS 8
-
 size_t lnb_trsm_f64_ws_bytes(int64_t n, int64_t nrhs)
 {
     const int64_t nb = ceil_div(n, TRSV_H);
-    const int64_t i1 = lnb_trsm_sync_ints(n, TRSV_H), i2 = lnb_trsm_tiles_ints(nrhs);
     return lnb_align256((size_t)nb * TRSV_H * TRSV_H * sizeof(double)) +
-           lnb_align256((size_t)(i1 > i2 ? i1 : i2) * sizeof(int)) + 512;
+           lnb_align256((size_t)lnb_trsm_tiles_ints(nrhs) * sizeof(int)) + 512;
 }
 
 /* op(T) X = alpha B with T triangular (uplo as stored), left side */
@@ -53,25 +47,17 @@ int lnb_trsm_f64_run(lnb_ctx *c, char uplo, char trans, char diag, int64_t n, in
         if (!dinv) return lnb_set_error(LNB_ENOMEM, "trsm workspace");
         CK(lnb_k_trtri_blocks_f64(dT, ldt, n, TRSV_H, uplo, diag == 'U', dinv, s), "trtri");
     }
-    if (nrhs > TRSM_CHAIN_MAX_NRHS) {
-        int *sync = (int *)lnb_arena_take(ar, (size_t)lnb_trsm_tiles_ints(nrhs) * sizeof(int));
-        if (!sync) return lnb_set_error(LNB_ENOMEM, "trsm sync workspace");
-        CK(lnb_k_trsm_tiles_f64(uplo, trans, n, nrhs, alpha, dT, ldt, dinv, dB, ldb, sync, c->st, lnb_wait_ns(),
-                                c->sms, s), "trsm tiles");
-        return 0;
-    }
-    int *sync = (int *)lnb_arena_take(ar, (size_t)lnb_trsm_sync_ints(n, TRSV_H) * sizeof(int));
+    int *sync = (int *)lnb_arena_take(ar, (size_t)lnb_trsm_tiles_ints(nrhs) * sizeof(int));
     if (!sync) return lnb_set_error(LNB_ENOMEM, "trsm sync workspace");
-    CK(lnb_k_trsm_left_f64(uplo, trans, n, nrhs, alpha, dT, ldt, dinv, TRSV_H, dB, ldb, sync, c->st,
-                           lnb_wait_ns(), 0, s), "trsm dag");
+    CK(lnb_k_trsm_tiles_f64(uplo, trans, n, nrhs, alpha, dT, ldt, dinv, dB, ldb, sync, c->st, lnb_wait_ns(), c->sms, 0,
+                            s), "trsm tiles");
     return 0;
 }
 
 int lnb_selftest_wait_timeout(long long wait_us)
 {
-    /* 1024 x 1024 identity, 1 rhs.  The ticket starts at 1, so no CTA walks
-     * the diagonal chain, and the off-band update items wait on solution
-     * blocks that nothing publishes. */
+    /* 1024 x 1024 identity, 1 rhs.  The ticket starts at 1, so the first block
+     * row is never solved and every other task waits for it. */
     lnb_ctx *c = lnb_ctx_get();
     if (!c) return LNB_ENODEV;
     const int64_t n = 1024;
@@ -80,14 +66,14 @@ int lnb_selftest_wait_timeout(long long wait_us)
     lnb_arena ar = {(char *)ws, 0, c->ws_size};
     double *T = lnb_arena_take(&ar, n * n * 8), *B = lnb_arena_take(&ar, n * 8);
     double *dinv = lnb_arena_take(&ar, (size_t)ceil_div(n, TRSV_H) * TRSV_H * TRSV_H * 8);
-    int *sync = lnb_arena_take(&ar, (size_t)lnb_trsm_sync_ints(n, TRSV_H) * sizeof(int));
+    int *sync = lnb_arena_take(&ar, (size_t)lnb_trsm_tiles_ints(1) * sizeof(int));
     cudaStream_t s = c->main;
     CK(cudaMemsetAsync(c->st, 0, sizeof(lnb_status_t), s), "status reset");
     CK(cudaMemsetAsync(T, 0, n * n * 8, s), "zero");
     CK(cudaMemsetAsync(B, 0, n * 8, s), "zero");
     CK(lnb_k_trtri_blocks_f64(T, n, n, TRSV_H, 'L', 1, dinv, s), "trtri");
-    CK(lnb_k_trsm_left_f64('L', 'N', n, 1, 1.0, T, n, dinv, TRSV_H, B, n, sync, c->st,
-                           (wait_us > 0 ? wait_us : 1000) * 1000LL, 1, s), "trsm dag");
+    CK(lnb_k_trsm_tiles_f64('L', 'N', n, 1, 1.0, T, n, dinv, B, n, sync, c->st, (wait_us > 0 ? wait_us : 1000) * 1000LL,
+                            c->sms, 1, s), "trsm tiles");
     return lnb_status_read(c, s);
 }
 
