@@ -256,13 +256,15 @@ LNB_DEV bool multiply(const Args &a, int v, int s, double *sm, Shared &sh, int &
     const int64_t oi = (int64_t)(a.fwd ? v : a.nb - 1 - v) * TS, c0 = (int64_t)s * NW;
     const int rows = blk_len(a, oi), cols = (int)(a.nrhs - c0 < NW ? a.nrhs - c0 : NW);
     double *Rs = sm, *Ds = sm + C::RING, *Bt = a.B + oi + c0 * a.ldb;
-    double acc[MI][NI][4];
+    // the sum over a tile's 64 terms, and over the tiles: one accumulator through up
+    // to n terms doubled the error of a solve with n = 8192
+    double acc[MI][NI][4], tot[MI][NI][4];
 #pragma unroll
     for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
         for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[mi][ni][e] = 0.0;
+            for (int e = 0; e < 4; ++e) acc[mi][ni][e] = tot[mi][ni][e] = 0.0;
     // B's own entries are fetched ahead of the last 64 terms and used after them
     double rhs[MI][NI][4];
     auto take_rhs = [&]() {
@@ -279,9 +281,10 @@ LNB_DEV bool multiply(const Args &a, int v, int s, double *sm, Shared &sh, int &
     };
     bool ok = true;
     const int nch = v * (TS / BK);
-    if (nch == 0) take_rhs();
+    // (64 columns: at the end, the registers hold the sums)
+    if (nch == 0 && NW < 64) take_rhs();
     for (int c = 0; c < nch; ++c) {
-        if (c == nch - TS / BK) take_rhs();
+        if (NW < 64 && c == nch - TS / BK) take_rhs();
         const int st = q % C::ST;
         if (!bar_wait(&sh.full[st], (q / C::ST) & 1, 4 * a.wait_ns, sh)) {
             ok = false;
@@ -307,8 +310,20 @@ LNB_DEV bool multiply(const Args &a, int v, int s, double *sm, Shared &sh, int &
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&sh.empty[st]);
         ++q;
+        if (c % (TS / BK) == TS / BK - 1) {
+#pragma unroll
+            for (int mi = 0; mi < MI; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < NI; ++ni)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        tot[mi][ni][e] += acc[mi][ni][e];
+                        acc[mi][ni][e] = 0.0;
+                    }
+        }
     }
     if (!mma_sync_and(ok)) return false;             // the ring is free
+    if (NW == 64) take_rhs();
 #pragma unroll
     for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
@@ -317,7 +332,7 @@ LNB_DEV bool multiply(const Args &a, int v, int s, double *sm, Shared &sh, int &
             for (int e = 0; e < 4; ++e) {
                 const int r = wm * (TS / WM) + mi * 16 + g + ((e & 2) ? 8 : 0);
                 const int c = wn * (NW / WN) + ni * 8 + 2 * t + (e & 1);
-                Rs[c * LDC + r] = fma(a.alpha, rhs[mi][ni][e], -acc[mi][ni][e]);
+                Rs[c * LDC + r] = fma(a.alpha, rhs[mi][ni][e], -tot[mi][ni][e]);
             }
     ok = bar_wait(&sh.dfull, nd & 1, 4 * a.wait_ns, sh);
     ++nd;
