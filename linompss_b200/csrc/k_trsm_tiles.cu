@@ -31,14 +31,16 @@
 namespace lnb {
 namespace tiles {
 
-constexpr int TS = 64, BK = 16, NT = 128, NTHR = NT + 32;
+constexpr int TS = 64, NT = 128, NTHR = NT + 32;
 constexpr int LDC = TS + 4;         // rows contiguous: S[k][m], ld = 4 mod 16 doubles
-constexpr int LDR = BK + 4;         // k contiguous: S[m][k], ld = 4 mod 16 doubles
-constexpr int ACH = TS * LDR;       // doubles of a staged chunk of op(T) (either layout)
-static_assert(BK * LDC <= ACH, "both layouts fit");
 
 template <int NW> struct Cfg {
-    static constexpr int ST = NW == 64 ? 3 : 4;
+    // chunks of 16 along k; 32 for the narrow strips, whose chain feels the per-chunk cost
+    static constexpr int BK = NW == 16 ? 32 : 16;
+    static constexpr int ST = NW == 32 ? 4 : 3;
+    static constexpr int LDR = BK + 4;             // k contiguous: S[m][k], ld = 4 mod 16 doubles
+    static constexpr int ACH = TS * LDR;           // doubles of a staged chunk of op(T) (either layout)
+    static_assert(BK * LDC <= ACH, "both layouts fit");
     static constexpr int STAGE = ACH + NW * LDR;
     static constexpr int RING = ST * STAGE;
     static_assert(NW * LDC <= RING, "the right-hand side of the diagonal product reuses the ring");
@@ -146,32 +148,33 @@ LNB_DEV void load64(double *dst, const double *X, int64_t ld, int nr, int nc, bo
         }
     }
 }
-// NC columns of 16 contiguous elements: dst[c * LDR + r] = X[r + c ld]
-template <int NC>
-LNB_DEV void load16(double *dst, const double *X, int64_t ld, int nr, int nc, bool vec, int lane)
+// NC columns of RUN (16 or 32) contiguous elements: dst[c * (RUN + 4) + r] = X[r + c ld]
+template <int RUN, int NC>
+LNB_DEV void load_run(double *dst, const double *X, int64_t ld, int nr, int nc, bool vec, int lane)
 {
+    constexpr int LDR = RUN + 4, CV = 64 / RUN, CE = 32 / RUN;     // columns per instruction
     if (vec) {
-        const int r = 2 * (lane & 7), bytes = r + 1 < nr ? 16 : r < nr ? 8 : 0;
-        int c = lane >> 3;
+        const int r = 2 * (lane & (RUN / 2 - 1)), bytes = r + 1 < nr ? 16 : r < nr ? 8 : 0;
+        int c = lane / (RUN / 2);
         uint32_t d = smem_u32(dst + c * LDR + r);
         const double *g = X + (bytes ? r : 0) + c * ld;
-        const int64_t step = 4 * ld;
+        const int64_t step = CV * ld;
         if (nc >= NC) {
 #pragma unroll
-            for (int it = 0; it < NC / 4; ++it, g += step) cp16(d + it * (4 * LDR * 8), g, bytes);
+            for (int it = 0; it < NC / CV; ++it, g += step) cp16(d + it * (CV * LDR * 8), g, bytes);
         } else {
 #pragma unroll 1
-            for (int it = 0; it < NC / 4; ++it, c += 4, d += 4 * LDR * 8, g += step)
+            for (int it = 0; it < NC / CV; ++it, c += CV, d += CV * LDR * 8, g += step)
                 cp16(d, c < nc ? g : X, c < nc ? bytes : 0);
         }
     } else {
-        const int r = lane & 15, bytes = r < nr ? 8 : 0;
-        int c = lane >> 4;
+        const int r = lane & (RUN - 1), bytes = r < nr ? 8 : 0;
+        int c = lane / RUN;
         uint32_t d = smem_u32(dst + c * LDR + r);
         const double *g = X + (bytes ? r : 0) + c * ld;
-        const int64_t step = 2 * ld;
+        const int64_t step = CE * ld;
 #pragma unroll 4
-        for (int it = 0; it < NC / 2; ++it, c += 2, d += 2 * LDR * 8, g += step) cp8(d, c < nc ? g : X, c < nc ? bytes : 0);
+        for (int it = 0; it < NC / CE; ++it, c += CE, d += CE * LDR * 8, g += step) cp8(d, c < nc ? g : X, c < nc ? bytes : 0);
     }
 }
 
@@ -182,6 +185,7 @@ template <int NW, bool TR>
 LNB_DEV bool produce(const Args &a, int v, int s, double *sm, Shared &sh, int &q)
 {
     using C = Cfg<NW>;
+    constexpr int BK = C::BK;
     const int lane = threadIdx.x & 31;
     const bool vt = ((uintptr_t)a.T % 16 == 0) && a.ldt % 2 == 0;
     const bool vb = ((uintptr_t)a.B % 16 == 0) && a.ldb % 2 == 0;
@@ -208,12 +212,12 @@ LNB_DEV bool produce(const Args &a, int v, int s, double *sm, Shared &sh, int &q
             const int kn = kt - c * BK < 0 ? 0 : kt - c * BK < BK ? kt - c * BK : BK;
             double *as = sm + st * C::STAGE;
             if (!TR) load64<BK>(as, kn ? Tu + c * BK * a.ldt : a.T, a.ldt, rows, kn, vt, lane);
-            else load16<TS>(as, kn ? Tu + c * BK : a.T, a.ldt, kn, rows, vt, lane);
+            else load_run<BK, TS>(as, kn ? Tu + c * BK : a.T, a.ldt, kn, rows, vt, lane);
         };
         auto load_b = [&](int c) {
             const int st = (q + c) % C::ST;
             const int kn = kt - c * BK < 0 ? 0 : kt - c * BK < BK ? kt - c * BK : BK;
-            load16<NW>(sm + st * C::STAGE + ACH, kn ? Bu + c * BK : a.B, a.ldb, kn, cols, vb, lane);
+            load_run<BK, NW>(sm + st * C::STAGE + C::ACH, kn ? Bu + c * BK : a.B, a.ldb, kn, cols, vb, lane);
             arrive_copied(&sh.full[st]);
         };
         int ahead = 0;                               // chunks whose part of T goes out before the wait
@@ -249,6 +253,7 @@ template <int NW, bool TR>
 LNB_DEV bool multiply(const Args &a, int v, int s, double *sm, Shared &sh, int &q, int &nd)
 {
     using C = Cfg<NW>;
+    constexpr int BK = C::BK, LDR = C::LDR;
     constexpr int WN = NW == 64 ? 2 : 1, WM = 4 / WN;       // warp grid of the sum
     constexpr int MI = TS / WM / 16, NI = NW / WN / 8;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -290,7 +295,7 @@ LNB_DEV bool multiply(const Args &a, int v, int s, double *sm, Shared &sh, int &
             ok = false;
             break;
         }
-        const double *as = sm + st * C::STAGE, *bs = as + ACH + (wn * (NW / WN) + g) * LDR + t;
+        const double *as = sm + st * C::STAGE, *bs = as + C::ACH + (wn * (NW / WN) + g) * LDR + t;
 #pragma unroll
         for (int kq = 0; kq < BK / 4; ++kq) {
             double a0[MI], a1[MI], b0[NI];
