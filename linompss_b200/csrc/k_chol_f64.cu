@@ -301,61 +301,102 @@ __global__ void __launch_bounds__(128) k_trsm_rlt_f64(const double *__restrict__
 // ========================================================================
 // C = alpha op(A) op(B) + beta C, optionally restricted to a triangle of C
 // (tri = 'L' or 'U'), on DMMA: 64 x 64 CTA tiles, 4 warps of 32 x 32, BK = 16,
-// 4-stage cp.async pipeline, two CTAs per SM.  Each operand is staged in the
+// cp.async pipeline, three CTAs per SM.  Each operand is staged in the
 // orientation its memory is contiguous in, so every copy is a 16-byte
 // cp.async along a column: op(A) = A and op(B) = B^T are stored k-major
 // (S[k][m], row stride 68), op(A) = A^T and op(B) = B m-major (S[m][k], row
 // stride 20).  Both strides spread a half-warp's fragment reads over all 32
 // banks.  beta == 0 does not read C (BLAS semantics).
+// Bound by the DMMA rate.  A thread's places in a chunk are the same for every
+// chunk, so its pointers and its rows' predicates are set once and a chunk costs
+// four copies per operand; with them computed per copy two CTAs per SM fitted and
+// the n = k = 4000 SYRK ran at 26.4 TF/s, now 31.1 (8192: 29.4, now 33.5).
 namespace gm {
-constexpr int BM = 64, BN = 64, BK = 16, ST = 4, THREADS = 128;
+constexpr int BM = 64, BN = 64, BK = 16, THREADS = 128;
 constexpr int LDKM = BM + 4;                  // k-major row stride (doubles)
 constexpr int LDMK = BK + 4;                  // m-major row stride
-constexpr int STAGE = (BM * LDMK > BK * LDKM) ? BM * LDMK : BK * LDKM;
-constexpr int SMEM = ST * 2 * STAGE * (int)sizeof(double);
+template <bool KM> constexpr int opsize() { return KM ? BK * LDKM : BM * LDMK; }
+template <bool AKM, bool BKM> struct Cfg {
+    static constexpr int ST = 3;                                    // three CTAs in an SM's shared memory
+    static constexpr int STAGE = opsize<AKM>() + opsize<BKM>();
+    static constexpr int SMEM = ST * STAGE * (int)sizeof(double);
+};
 
-// two consecutive elements src[0], src[1] (nv of them valid) -> dst[0..1]
-LNB_DEV void load2(double *dst, const double *src, int nv)
-{
-    if (nv == 2 && ((uintptr_t)src & 15) == 0) {
-        cp_async16(dst, src, true);
-    } else {
-        cp_async8(dst, nv > 0 ? src : dst, nv > 0);
-        cp_async8(dst + 1, nv > 1 ? src + 1 : dst, nv > 1);
-    }
-}
-
-// rows x BK tile of an operand whose element (r, k) is X[r + k ldx] (KM:
-// contiguous in r -> k-major smem) or X[k + r ldx] (!KM: contiguous in k ->
-// r-major smem); rows [r0, r0 + 64) of nr, k in [k0, k0 + BK) of nk
+// One thread's share of an operand's chunks: four places, 16 bytes each.  Element
+// (r, k) of the operand is X[r + k ldx] (KM) or X[k + r ldx]; rows [r0, r0 + 64) of
+// nr, k of nk.
 template <bool KM>
-LNB_DEV void load_op(double *dst, const double *X, int64_t ldx, int64_t r0, int64_t nr, int64_t k0, int64_t nk,
-                     int tid)
-{
-#pragma unroll
-    for (int it = 0; it < (BM * BK / 2) / THREADS; ++it) {
-        const int idx = tid + it * THREADS;
+struct Loader {
+    const double *g;            // the first place in the current chunk
+    const double *safe;         // readable address for copies of zero bytes
+    int64_t step, ldx;          // between places; between chunks (KM: BK ldx)
+    int kk, nk;                 // k of the first place; all k
+    int bytes[4];               // valid bytes of each place (0, 8, 16), rows only
+    uint32_t off;               // byte offset of the first place in a stage
+    bool vec;
+    LNB_DEV Loader(const double *X, int64_t ldx_, int64_t r0, int64_t nr, int64_t nk_)
+    {
+        const int tid = threadIdx.x;
+        vec = ((uintptr_t)X & 15) == 0 && (ldx_ & 1) == 0;
+        nk = (int)nk_;
+        ldx = ldx_;
+        safe = X;
         if (KM) {
-            const int kk = idx / (BM / 2), rr = (idx % (BM / 2)) * 2;
-            const int64_t r = r0 + rr, k = k0 + kk;
-            const int nv = k < nk ? (int)(r + 1 < nr ? 2 : (r < nr ? 1 : 0)) : 0;
-            load2(dst + kk * LDKM + rr, X + (nv ? r + k * ldx : 0), nv);
+            const int rr = (tid & 31) * 2;
+            kk = tid >> 5;                          // + 4 it
+            const int v = r0 + rr + 1 < nr ? 16 : r0 + rr < nr ? 8 : 0;
+            g = X + (v ? r0 + rr : 0) + kk * ldx;
+            step = 4 * ldx;
+#pragma unroll
+            for (int it = 0; it < 4; ++it) bytes[it] = v;
+            off = (uint32_t)(kk * LDKM + rr) * 8;
         } else {
-            const int rr = idx / (BK / 2), kk = (idx % (BK / 2)) * 2;
-            const int64_t r = r0 + rr, k = k0 + kk;
-            const int nv = r < nr ? (int)(k + 1 < nk ? 2 : (k < nk ? 1 : 0)) : 0;
-            load2(dst + rr * LDMK + kk, X + (nv ? k + r * ldx : 0), nv);
+            const int rr = tid >> 3;                // + 16 it
+            kk = (tid & 7) * 2;
+            g = X + (r0 + rr) * ldx + kk;
+            step = 16 * ldx;
+#pragma unroll
+            for (int it = 0; it < 4; ++it) bytes[it] = r0 + rr + 16 * it < nr ? 16 : 0;
+            off = (uint32_t)(rr * LDMK + kk) * 8;
         }
     }
-}
+    // the chunk at k0 (a multiple of BK, in ascending order) into the stage at s
+    LNB_DEV void load(uint32_t s, int k0)
+    {
+        constexpr uint32_t ds = (KM ? 4 * LDKM : 16 * LDMK) * 8;
+        s += off;
+        const bool full = k0 + BK <= nk;
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+            const double *p = g + it * step;
+            int n = bytes[it];
+            if (!full) {
+                if (KM) n = k0 + kk + 4 * it < nk ? n : 0;
+                else n = k0 + kk + 1 < nk ? n : k0 + kk < nk ? (n ? 8 : 0) : 0;
+            }
+            p = n ? p : safe;
+            if (vec) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s + it * ds), "l"(p), "r"(n));
+            } else {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s + it * ds), "l"(p),
+                             "r"(n > 0 ? 8 : 0));
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s + it * ds + 8),
+                             "l"(n > 8 ? p + 1 : safe), "r"(n > 8 ? 8 : 0));
+            }
+        }
+        g += KM ? BK * ldx : BK;
+    }
+};
 
 // AKM: op(A) = A (k-major staging); BKM: op(B) = B^T (k-major staging)
 template <bool AKM, bool BKM>
-__global__ void __launch_bounds__(THREADS, 2) k_gemm_dmma(int64_t M, int64_t N, int64_t K, double alpha,
+__global__ void __launch_bounds__(THREADS, 3) k_gemm_dmma(int64_t M, int64_t N, int64_t K, double alpha,
                                                           const double *__restrict__ A, int64_t lda,
                                                           const double *__restrict__ B, int64_t ldb, double beta,
                                                           double *C, int64_t ldc, char tri)
 {
+    using Cf = Cfg<AKM, BKM>;
+    constexpr int ST = Cf::ST;
     const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
     if (tri == 'L' && m0 + BM <= n0) return;
     if (tri == 'U' && n0 + BN <= m0) return;
@@ -363,10 +404,12 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemm_dmma(int64_t M, int64_t N, 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wm = warp >> 1, wn = warp & 1, g = lane >> 2, t = lane & 3;
     const int ktiles = (int)((K + BK - 1) / BK);
+    Loader<AKM> la(A, lda, m0, M, K);
+    Loader<BKM> lb(B, ldb, n0, N, K);
+    const uint32_t s0 = smem_u32(gsm);
     auto stage = [&](int s, int kt) {
-        double *as = gsm + (2 * s) * STAGE, *bs = gsm + (2 * s + 1) * STAGE;
-        load_op<AKM>(as, A, lda, m0, M, (int64_t)kt * BK, K, tid);
-        load_op<BKM>(bs, B, ldb, n0, N, (int64_t)kt * BK, K, tid);
+        la.load(s0 + s * (Cf::STAGE * 8), kt * BK);
+        lb.load(s0 + s * (Cf::STAGE * 8) + opsize<AKM>() * 8, kt * BK);
     };
     double acc[2][4][4];
 #pragma unroll
@@ -380,15 +423,15 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemm_dmma(int64_t M, int64_t N, 
         if (s < ktiles) stage(s, s);
         cp_async_commit();
     }
+    int rd = 0, wr = ST - 1;                       // stages read and written
     for (int kt = 0; kt < ktiles; ++kt) {
         cp_async_wait<ST - 2>();
         __syncthreads();
-        {
-            const int nk = kt + ST - 1;
-            if (nk < ktiles) stage(nk % ST, nk);
-            cp_async_commit();
-        }
-        const double *as = gsm + (2 * (kt % ST)) * STAGE, *bs = gsm + (2 * (kt % ST) + 1) * STAGE;
+        if (kt + ST - 1 < ktiles) stage(wr, kt + ST - 1);
+        cp_async_commit();
+        const double *as = gsm + rd * Cf::STAGE, *bs = as + opsize<AKM>();
+        rd = rd + 1 == ST ? 0 : rd + 1;
+        wr = wr + 1 == ST ? 0 : wr + 1;
 #pragma unroll
         for (int kq = 0; kq < BK / 4; ++kq) {
             const int k = kq * 4 + t;
@@ -411,20 +454,28 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemm_dmma(int64_t M, int64_t N, 
         }
     }
     cp_async_wait<0>();
+    // sixteen loads of C in flight: through one pointer the compiler would finish
+    // each read-modify-write before the next
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
+    for (int mi = 0; mi < 2; ++mi) {
+        const int64_t r0 = m0 + wm * 32 + mi * 16 + g, c0 = n0 + wn * 32 + 2 * t;
+        double *cp = C + r0 + c0 * ldc;
+        auto keep = [&](int ni, int q) {
+            const int64_t r = r0 + (q >> 1) * 8, c = c0 + ni * 8 + (q & 1);
+            return r < M && c < N && !(tri == 'L' && r < c) && !(tri == 'U' && r > c);
+        };
+        double cv[4][4];
 #pragma unroll
         for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int64_t r = m0 + wm * 32 + mi * 16 + g + (q >> 1) * 8;
-                const int64_t c = n0 + wn * 32 + ni * 8 + 2 * t + (q & 1);
-                if (r >= M || c >= N) continue;
-                if (tri == 'L' && r < c) continue;
-                if (tri == 'U' && r > c) continue;
-                double *cp = &C[r + c * ldc];
-                *cp = (beta == 0.0 ? 0.0 : beta * *cp) + alpha * acc[mi][ni][q];
-            }
+            for (int q = 0; q < 4; ++q)
+                cv[ni][q] = beta != 0.0 && keep(ni, q) ? beta * cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] : 0.0;
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (keep(ni, q)) cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] = cv[ni][q] + alpha * acc[mi][ni][q];
+    }
 }
 }  // namespace gm
 
@@ -504,11 +555,12 @@ static void launch_gemm(int64_t m, int64_t n, int64_t k, double alpha, const dou
 {
     static bool attr = false;
     if (!attr) {
-        cudaFuncSetAttribute(gm::k_gemm_dmma<AKM, BKM>, cudaFuncAttributeMaxDynamicSharedMemorySize, gm::SMEM);
+        cudaFuncSetAttribute(gm::k_gemm_dmma<AKM, BKM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             gm::Cfg<AKM, BKM>::SMEM);
         attr = true;
     }
     dim3 grid((unsigned)((n + gm::BN - 1) / gm::BN), (unsigned)((m + gm::BM - 1) / gm::BM));
-    gm::k_gemm_dmma<AKM, BKM><<<grid, gm::THREADS, gm::SMEM, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
+    gm::k_gemm_dmma<AKM, BKM><<<grid, gm::THREADS, gm::Cfg<AKM, BKM>::SMEM, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
                                                                   tri);
 }
 
