@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(THREADS, 3) k_gemm_dmma(int64_t M, int64_t N, 
         for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                if (keep(ni, q)) cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] = cv[ni][q] + alpha * acc[mi][ni][q];
+                if (keep(ni, q)) cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] = __dadd_rn(cv[ni][q], __dmul_rn(alpha, acc[mi][ni][q]));
     }
 }
 }  // namespace gm

@@ -229,21 +229,6 @@ static int check_args(int n, int b, const void *A, int lda)
 
 static inline int64_t ld_dev(int64_t n) { return (n + 7) & ~(int64_t)7; }
 
-/* copy the lower block-columns (step columns each, rows from the block's
- * first column down) of a column-major matrix host<->device.  With step = b
- * every diagonal tile travels whole, which the panel copy-back relies on. */
-static int copy_lower(double *dst, int64_t ldd, const double *src, int64_t lds, int64_t n,
-                      int64_t step, enum cudaMemcpyKind kind, cudaStream_t s)
-{
-    for (int64_t c0 = 0; c0 < n; c0 += step) {
-        int64_t w = n - c0 < step ? n - c0 : step;
-        CK(cudaMemcpy2DAsync(dst + c0 + c0 * ldd, (size_t)ldd * sizeof(double), src + c0 + c0 * lds,
-                             (size_t)lds * sizeof(double), (size_t)(n - c0) * sizeof(double), (size_t)w,
-                             kind, s), "copy");
-    }
-    return 0;
-}
-
 static int chol_host(int n, int b, double *A, int lda)
 {
     int e = check_args(n, b, A, lda);
@@ -258,10 +243,10 @@ static int chol_host(int n, int b, double *A, int lda)
     lnb_arena ar = {(char *)ws, 0, c->ws_size};
     double *dA = (double *)lnb_arena_take(&ar, abytes);
     cudaStream_t s = c->main;
-    if ((e = copy_lower(dA, ldd, A, lda, n, b, cudaMemcpyHostToDevice, s))) return e;
+    if ((e = lnb_copy_lower_f64(c, dA, ldd, A, lda, n, b, 1, s))) return e;
     const int pinned = lnb_host_is_pinned(A);
     if ((e = lnb_chol_f64_run_w(c, n, b, dA, ldd, &ar, s, pinned ? A : NULL, lda, NULL))) return e;
-    if (!pinned && (e = copy_lower(A, lda, dA, ldd, n, b, cudaMemcpyDeviceToHost, s))) return e;
+    if (!pinned && (e = lnb_copy_lower_f64(c, dA, ldd, A, lda, n, b, 0, s))) return e;
     return lnb_status_read(c, s);
 }
 

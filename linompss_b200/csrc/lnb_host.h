@@ -16,6 +16,7 @@ extern "C" {
 #endif
 
 /* per-device context: streams, events, cached workspace, status words */
+#define LNB_STAGE_SLOTS 8
 typedef struct {
     int           ready;
     int           device;
@@ -30,6 +31,8 @@ typedef struct {
     lnb_status_t *st;          /* device status word */
     lnb_status_t *st_host;     /* pinned host mirror */
     cudaEvent_t   t0, t1;      /* timing */
+    void         *stage;       /* pinned slots of the pageable copies (lnb_stage.c) */
+    cudaEvent_t   stage_ev[LNB_STAGE_SLOTS];
 } lnb_ctx;
 
 /* Returns the current device's context (creating it), or NULL after setting
@@ -48,6 +51,19 @@ static inline void *lnb_arena_take(lnb_arena *a, size_t bytes)
     a->off = o + bytes;
     return a->base + o;
 }
+
+/* Copies between host matrices and the device, columns of `width` bytes
+ * (lnb_stage.c).  Pageable host memory: the host part is done when the call
+ * returns; otherwise as cudaMemcpy2DAsync on s.  0 or LNB_E*. */
+typedef struct { char *dev, *host; size_t width, cols; } lnb_rect;
+int lnb_copy_rects(lnb_ctx *c, const lnb_rect *r, int nr, size_t dpitch, size_t hpitch, int to_device,
+                   cudaStream_t s, const char *where);
+int lnb_copy_matrix(lnb_ctx *c, void *dev, size_t dpitch, const void *host, size_t hpitch, size_t width, size_t cols,
+                    int to_device, cudaStream_t s, const char *where);
+/* the lower block columns (step columns each, rows from the block's first column down) */
+int lnb_copy_lower_f64(lnb_ctx *c, double *dev, int64_t ldd, const double *host, int64_t ldh, int64_t n, int64_t step,
+                       int to_device, cudaStream_t s);
+void lnb_stage_release(lnb_ctx *c);
 
 int  lnb_set_error(int code, const char *fmt, ...);
 int  lnb_cuda_error(int cuda_err, const char *where);

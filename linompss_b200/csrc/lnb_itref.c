@@ -103,13 +103,6 @@ static int dcg_dev(lnb_ctx *c, int64_t n, const double *dA, int64_t lda, const d
     return k;
 }
 
-static int copy_in_matrix(double *d, int64_t ldd, const double *h, int64_t ldh, int64_t n, cudaStream_t s)
-{
-    CK(cudaMemcpy2DAsync(d, (size_t)ldd * 8, h, (size_t)ldh * 8, (size_t)n * 8, (size_t)n,
-                         cudaMemcpyHostToDevice, s), "A in");
-    return 0;
-}
-
 int ompss_dcg(int n, int bm, const double *A, int lda, const double *b, double *x, double tol, int steps)
 {
     (void)bm;
@@ -128,7 +121,7 @@ int ompss_dcg(int n, int bm, const double *A, int lda, const double *b, double *
     int e;
     if ((e = cg_ws_take(&ar, n, c->sms, &w))) return e;
     cudaStream_t s = c->main;
-    if ((e = copy_in_matrix(dA, ldd, A, lda, n, s))) return e;
+    if ((e = lnb_copy_matrix(c, dA, (size_t)ldd * 8, A, (size_t)lda * 8, (size_t)n * 8, (size_t)n, 1, s, "A in"))) return e;
     CK(cudaMemcpyAsync(db, b, (size_t)n * 8, cudaMemcpyHostToDevice, s), "b in");
     CK(cudaMemcpyAsync(dx, x, (size_t)n * 8, cudaMemcpyHostToDevice, s), "x in");
     int rc = dcg_dev(c, n, dA, ldd, db, dx, tol, steps, 0, &w, s);
@@ -164,7 +157,7 @@ int ompss_ditref(int n, int bm, const double *A, int lda, const double *b, doubl
     int e;
     if ((e = cg_ws_take(&ar, n, c->sms, &w))) return e;
     cudaStream_t s = c->main;
-    if ((e = copy_in_matrix(dA, ldd, A, lda, n, s))) return e;
+    if ((e = lnb_copy_matrix(c, dA, (size_t)ldd * 8, A, (size_t)lda * 8, (size_t)n * 8, (size_t)n, 1, s, "A in"))) return e;
     CK(cudaMemcpyAsync(rhs, b, (size_t)n * 8, cudaMemcpyHostToDevice, s), "b in");
     CK(cudaMemsetAsync(sd[1], 0, (size_t)n * 8, s), "zero");
     /* initial solve from x = 0 (itref.c:1001-1006) */

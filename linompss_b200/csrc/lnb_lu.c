@@ -127,33 +127,23 @@ static int getrs_run(lnb_ctx *c, int64_t n, int64_t nrhs, const double *dLU, int
 static inline int64_t ld_dev(int64_t m) { return (m + 7) & ~(int64_t)7; }
 
 /* host matrix (m x n, ld, FP64 or FP32) -> device FP64 (ld ldd) */
-static int mat_in(double *d, int64_t ldd, const void *h, int64_t ld, int64_t m, int64_t n, float *f32,
+static int mat_in(lnb_ctx *c, double *d, int64_t ldd, const void *h, int64_t ld, int64_t m, int64_t n, float *f32,
                   cudaStream_t s)
 {
     if (m <= 0 || n <= 0) return 0;
-    if (!f32) {
-        CK(cudaMemcpy2DAsync(d, (size_t)ldd * 8, h, (size_t)ld * 8, (size_t)m * 8, n, cudaMemcpyHostToDevice, s),
-           "matrix in");
-    } else {
-        CK(cudaMemcpy2DAsync(f32, (size_t)m * 4, h, (size_t)ld * 4, (size_t)m * 4, n, cudaMemcpyHostToDevice, s),
-           "matrix in");
-        CK(lnb_k_f32_to_f64(f32, m, m, n, d, ldd, s), "widen");
-    }
+    if (!f32) return lnb_copy_matrix(c, d, (size_t)ldd * 8, h, (size_t)ld * 8, (size_t)m * 8, n, 1, s, "matrix in");
+    const int e = lnb_copy_matrix(c, f32, (size_t)m * 4, h, (size_t)ld * 4, (size_t)m * 4, n, 1, s, "matrix in");
+    if (e) return e;
+    CK(lnb_k_f32_to_f64(f32, m, m, n, d, ldd, s), "widen");
     return 0;
 }
-static int mat_out(void *h, int64_t ld, const double *d, int64_t ldd, int64_t m, int64_t n, float *f32,
+static int mat_out(lnb_ctx *c, void *h, int64_t ld, const double *d, int64_t ldd, int64_t m, int64_t n, float *f32,
                    cudaStream_t s)
 {
     if (m <= 0 || n <= 0) return 0;
-    if (!f32) {
-        CK(cudaMemcpy2DAsync(h, (size_t)ld * 8, d, (size_t)ldd * 8, (size_t)m * 8, n, cudaMemcpyDeviceToHost, s),
-           "matrix out");
-    } else {
-        CK(lnb_k_f64_to_f32(d, ldd, m, n, f32, m, s), "narrow");
-        CK(cudaMemcpy2DAsync(h, (size_t)ld * 4, f32, (size_t)m * 4, (size_t)m * 4, n, cudaMemcpyDeviceToHost, s),
-           "matrix out");
-    }
-    return 0;
+    if (!f32) return lnb_copy_matrix(c, (void *)d, (size_t)ldd * 8, h, (size_t)ld * 8, (size_t)m * 8, n, 0, s, "matrix out");
+    CK(lnb_k_f64_to_f32(d, ldd, m, n, f32, m, s), "narrow");
+    return lnb_copy_matrix(c, f32, (size_t)m * 4, h, (size_t)ld * 4, (size_t)m * 4, n, 0, s, "matrix out");
 }
 
 static int getrf_host(int m, int n, int b, void *A, int lda, int *IPIV, int single)
@@ -176,9 +166,9 @@ static int getrf_host(int m, int n, int b, void *A, int lda, int *IPIV, int sing
     cudaStream_t s = c->main;
     int e;
     CK(cudaMemsetAsync(c->st, 0, sizeof(lnb_status_t), s), "status reset");
-    if ((e = mat_in(dA, ldd, A, lda, m, n, f32, s))) return e;
+    if ((e = mat_in(c, dA, ldd, A, lda, m, n, f32, s))) return e;
     if ((e = getrf_run(c, m, n, dA, ldd, dpiv, &ar, s))) return e;
-    if ((e = mat_out(A, lda, dA, ldd, m, n, f32, s))) return e;
+    if ((e = mat_out(c, A, lda, dA, ldd, m, n, f32, s))) return e;
     CK(cudaMemcpyAsync(IPIV, dpiv, pbytes, cudaMemcpyDeviceToHost, s), "pivots out");
     const int info = lnb_status_read(c, s);
     if (info < 0) return info;
@@ -221,13 +211,13 @@ static int gensolv_host(int m, int n, int b, void *A, void *B, int single)
     cudaStream_t s = c->main;
     int e;
     CK(cudaMemsetAsync(c->st, 0, sizeof(lnb_status_t), s), "status reset");
-    if ((e = mat_in(dA, ldd, A, m, m, m, f32, s))) return e;
+    if ((e = mat_in(c, dA, ldd, A, m, m, m, f32, s))) return e;
     if ((e = getrf_run(c, m, m, dA, ldd, dpiv, &ar, s))) return e;
-    if ((e = mat_out(A, m, dA, ldd, m, m, f32, s))) return e;
+    if ((e = mat_out(c, A, m, dA, ldd, m, m, f32, s))) return e;
     if (n > 0) {
-        if ((e = mat_in(dB, ldd, B, m, m, n, f32, s))) return e;
+        if ((e = mat_in(c, dB, ldd, B, m, m, n, f32, s))) return e;
         if ((e = getrs_run(c, m, n, dA, ldd, dpiv, dB, ldd, &ar, s))) return e;
-        if ((e = mat_out(B, m, dB, ldd, m, n, f32, s))) return e;
+        if ((e = mat_out(c, B, m, dB, ldd, m, n, f32, s))) return e;
     }
     return lnb_status_read(c, s);
 }

@@ -117,6 +117,7 @@ void lnb_release_workspace(void)
         c->ws = NULL;
         c->ws_size = 0;
     }
+    if (c->ready) lnb_stage_release(c);
 }
 
 int lnb_status_read(lnb_ctx *c, cudaStream_t s)

@@ -190,20 +190,15 @@ int dspdsolv_main(int m, int nrhs, int b, double *A, double *B)
     double *dA = (double *)lnb_arena_take(&ar, abytes);
     double *dB = (double *)lnb_arena_take(&ar, bbytes);
     cudaStream_t s = c->main;
-    /* lower block-columns of A, all of B */
-    for (int64_t c0 = 0; c0 < m; c0 += b) {
-        int64_t w = m - c0 < b ? m - c0 : b;
-        CK(cudaMemcpy2DAsync(dA + c0 + c0 * ldd, ldd * sizeof(double), A + c0 + c0 * (int64_t)m,
-                             (size_t)m * sizeof(double), (size_t)(m - c0) * sizeof(double), w,
-                             cudaMemcpyHostToDevice, s), "A in");
-    }
-    if (nrhs > 0)
-        CK(cudaMemcpy2DAsync(dB, ldd * sizeof(double), B, (size_t)m * sizeof(double),
-                             (size_t)m * sizeof(double), nrhs, cudaMemcpyHostToDevice, s), "B in");
+    /* lower block-columns of A (whole diagonal tiles), all of B */
+    int e;
+    if ((e = lnb_copy_lower_f64(c, dA, ldd, A, m, m, b, 1, s))) return e;
+    if (nrhs > 0 && (e = lnb_copy_matrix(c, dB, ldd * sizeof(double), B, (size_t)m * sizeof(double),
+                                         (size_t)m * sizeof(double), nrhs, 1, s, "B in")))
+        return e;
     const int pinned = lnb_host_is_pinned(A);
     double *dinv = NULL;
-    int e = lnb_chol_f64_run_w(c, m, b, dA, ldd, &ar, s, pinned ? A : NULL, m, &dinv);
-    if (e) return e;
+    if ((e = lnb_chol_f64_run_w(c, m, b, dA, ldd, &ar, s, pinned ? A : NULL, m, &dinv))) return e;
     if (nrhs > 0) {
         if (!dinv) {
             const int64_t nb = ceil_div(m, TRSV_H);
@@ -213,16 +208,11 @@ int dspdsolv_main(int m, int nrhs, int b, double *A, double *B)
         }
         if ((e = lnb_trsm_f64_run(c, 'L', 'N', 'N', m, nrhs, 1.0, dA, ldd, dB, ldd, &ar, s, dinv))) return e;
         if ((e = lnb_trsm_f64_run(c, 'L', 'T', 'N', m, nrhs, 1.0, dA, ldd, dB, ldd, &ar, s, dinv))) return e;
-        CK(cudaMemcpy2DAsync(B, (size_t)m * sizeof(double), dB, ldd * sizeof(double),
-                             (size_t)m * sizeof(double), nrhs, cudaMemcpyDeviceToHost, s), "X out");
+        if ((e = lnb_copy_matrix(c, dB, ldd * sizeof(double), B, (size_t)m * sizeof(double), (size_t)m * sizeof(double),
+                                 nrhs, 0, s, "X out")))
+            return e;
     }
-    if (!pinned)
-        for (int64_t c0 = 0; c0 < m; c0 += b) {
-            int64_t w = m - c0 < b ? m - c0 : b;
-            CK(cudaMemcpy2DAsync(A + c0 + c0 * (int64_t)m, (size_t)m * sizeof(double), dA + c0 + c0 * ldd,
-                                 ldd * sizeof(double), (size_t)(m - c0) * sizeof(double), w,
-                                 cudaMemcpyDeviceToHost, s), "L out");
-        }
+    if (!pinned && (e = lnb_copy_lower_f64(c, dA, ldd, A, m, m, b, 0, s))) return e;
     return lnb_status_read(c, s);
 }
 
@@ -250,13 +240,15 @@ int ompss_dtrsm(ompssblas_t side, ompssblas_t uplo, ompssblas_t trans, ompssblas
     double *dB = (double *)lnb_arena_take(&ar, bbytes);
     cudaStream_t s = c->main;
     CK(cudaMemsetAsync(c->st, 0, sizeof(lnb_status_t), s), "status reset");
-    CK(cudaMemcpy2DAsync(dA, ldd * sizeof(double), A, (size_t)lda * sizeof(double), (size_t)m * sizeof(double),
-                         m, cudaMemcpyHostToDevice, s), "A in");
-    CK(cudaMemcpy2DAsync(dB, ldd * sizeof(double), B, (size_t)ldb * sizeof(double), (size_t)m * sizeof(double),
-                         n, cudaMemcpyHostToDevice, s), "B in");
+    if ((e = lnb_copy_matrix(c, dA, ldd * sizeof(double), A, (size_t)lda * sizeof(double), (size_t)m * sizeof(double), m, 1,
+                             s, "A in")) ||
+        (e = lnb_copy_matrix(c, dB, ldd * sizeof(double), B, (size_t)ldb * sizeof(double), (size_t)m * sizeof(double), n, 1,
+                             s, "B in")))
+        return e;
     if ((e = lnb_trsm_f64_run(c, cu, ct, cd, m, n, alpha, dA, ldd, dB, ldd, &ar, s, NULL))) return e;
-    CK(cudaMemcpy2DAsync(B, (size_t)ldb * sizeof(double), dB, ldd * sizeof(double), (size_t)m * sizeof(double),
-                         n, cudaMemcpyDeviceToHost, s), "B out");
+    if ((e = lnb_copy_matrix(c, dB, ldd * sizeof(double), B, (size_t)ldb * sizeof(double), (size_t)m * sizeof(double), n, 0,
+                             s, "B out")))
+        return e;
     e = lnb_status_read(c, s);
     return e < 0 ? e : 0;
 }
