@@ -156,7 +156,7 @@ __global__ void k_cg_p(int64_t n, int mode, const double *num, const double *den
 // so the scalars agree to the last bit without being exchanged; only the product
 // A p is shared out, in tiles of 32 rows x a slab of columns, each leaving 32
 // partial sums.  All sums have a fixed shape: repeated runs are bit-identical.
-// Bound by latency up to a few thousand unknowns (n = 1500: 6 us a step, the matrix
+// Bound by latency up to a few thousand unknowns (n = 1500: 9 us a step, the matrix
 // in L2; as four launches and a host read per step it took 60), by the read of A
 // above.
 constexpr int CG_NT = 512, CG_NW = CG_NT / 32, CG_RG = 32;

@@ -115,6 +115,13 @@ LNB_DEV double pivot_rcp(double x)
     return fma(y, fma(e, e, e), y);
 }
 
+// The panel.  Bound by latency: each column is a pivot search over all rows, a row
+// broadcast and a rank-1 step, one after another.  A thread holds whole rows of the
+// panel in registers (moved down one place per column, so indexes stay constant),
+// one block barrier per column (a cluster barrier when the rows need several CTAs),
+// and the next column's search runs on its freshly updated values before the rest
+// of the row is updated.  16 columns of 1500 rows take 32 us, of 512 rows 17 us
+// (32 columns took 130 us by one CTA with the panel in shared memory).
 template <int NB, int RPT>
 __global__ void __launch_bounds__(PT, 1) k_lu_panel(double *A, int64_t lda, int64_t m, int64_t c0, int nb, int *piv,
                                                     Perm *perm, lnb_status_t *st)
@@ -302,7 +309,7 @@ __global__ void __launch_bounds__(PT, 1) k_lu_panel(double *A, int64_t lda, int6
 // than its barriers.  The update is one m16 x n8 DMMA strip of rows per warp at a
 // time, U in registers (the B fragments).  Bound by L2: every CTA reads the whole
 // panel; with the matrix in L2 and all columns right of the panel updated at once
-// a rank-16 step of n = 1500 takes 6 us.
+// a rank-16 step of n = 1500 takes 11 us.
 constexpr int AT = 256, AC = 8;
 template <int NB>
 __global__ void __launch_bounds__(AT) k_lu_apply(double *A, int64_t lda, int64_t m, int64_t c0, int nb,
@@ -616,23 +623,29 @@ extern "C" int lnb_k_laswp_f64(double *A, int64_t lda, int64_t k0, int64_t k1, c
     return (int)cudaGetLastError();
 }
 
+// largest n whose composed permutation fits a block's shared memory (getrs of factors made
+// elsewhere may have more rows than the panel kernel takes)
+extern "C" int64_t lnb_rows_permute_max(void) { return ((227 * 1024 - 32 * (int64_t)sizeof(Chunk)) / 4) & ~3ll; }
+
 // B (n rows, nrhs columns) takes the swaps k <-> piv[k]-1, k < k1 <= n; src: n
-// ints, T: n x nrhs doubles of scratch
+// ints, T: n x tcols doubles of scratch
 extern "C" int lnb_k_rows_permute_f64(double *B, int64_t ldb, int64_t n, int64_t nrhs, int64_t k1, const int *piv,
-                                      int *src, double *T, lnb_stream_t s)
+                                      int *src, double *T, int64_t tcols, lnb_stream_t s)
 {
     if (n <= 0 || nrhs <= 0 || k1 <= 0) return 0;
+    if (n > lnb_rows_permute_max()) return (int)cudaErrorInvalidValue;
     const int smem = (int)((n + 3) & ~3ll) * 4 + 32 * (int)sizeof(Chunk);
-    if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(k_piv_compose, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     k_piv_compose<<<1, 1024, smem, (cudaStream_t)s>>>((int)n, (int)k1, piv, src);
-    for (int64_t q = 0; q < nrhs; q += 65535) {
-        const int64_t nq = nrhs - q < 65535 ? nrhs - q : 65535;
+    lnb_prof_count(1);
+    const int64_t step = tcols < 65535 ? tcols : 65535;
+    for (int64_t q = 0; q < nrhs; q += step) {
+        const int64_t nq = nrhs - q < step ? nrhs - q : step;
         const dim3 grid((unsigned)((n + 255) / 256 < 64 ? (n + 255) / 256 : 64), (unsigned)nq);
-        k_rows_gather<<<grid, 256, 0, (cudaStream_t)s>>>(n, B + q * ldb, ldb, src, T + q * n);
-        k_rows_copy<<<grid, 256, 0, (cudaStream_t)s>>>(n, T + q * n, B + q * ldb, ldb);
+        k_rows_gather<<<grid, 256, 0, (cudaStream_t)s>>>(n, B + q * ldb, ldb, src, T);
+        k_rows_copy<<<grid, 256, 0, (cudaStream_t)s>>>(n, T, B + q * ldb, ldb);
+        lnb_prof_count(2);
     }
-    lnb_prof_count(3);
     return (int)cudaGetLastError();
 }

@@ -37,7 +37,7 @@ constexpr int NRC = 64;         // rhs columns per pass
 // diagonal blocks by forward substitution (a thread per column), then twice the
 // two-by-two step [A 0; C D]^-1 = [A^-1 0; -D^-1 C A^-1  D^-1], 16 -> 32 -> 64.
 // Bound by latency: the substitution over all 64 rows, a thread per column, was
-// 64 dependent rows of up to 64 terms and took 56 us; this takes 6.
+// 64 dependent rows of up to 64 terms and took 56 us (n = 8192, 128 blocks); this takes 20.
 constexpr int TI_NT = 256, TI_LD = TH + 1;
 // Z (h x h) = sum_k X[.][k] Y[k][.] of h x h blocks (row-major, ld TI_LD), sign s;
 // `part` of the CTA's threads: np threads, this one is p

@@ -50,8 +50,9 @@ int lnb_k_lu_apply_f64(double *A, int64_t lda, int64_t m, int64_t c0, int nb, co
                        int64_t a1, int64_t b0, int64_t b1, cudaStream_t s);
 int lnb_k_laswp_f64(double *A, int64_t lda, int64_t k0, int64_t k1, const int *piv, int64_t a0, int64_t a1,
                     int64_t b0, int64_t b1, cudaStream_t s);
+int64_t lnb_rows_permute_max(void);
 int lnb_k_rows_permute_f64(double *B, int64_t ldb, int64_t n, int64_t nrhs, int64_t k1, const int *piv, int *src,
-                           double *T, cudaStream_t s);
+                           double *T, int64_t tcols, cudaStream_t s);
 int lnb_k_f32_to_f64(const float *X, int64_t ldx, int64_t m, int64_t k, double *D, int64_t ldd, cudaStream_t st);
 int lnb_k_f64_to_f32(const double *D, int64_t ldd, int64_t m, int64_t k, float *X, int64_t ldx, cudaStream_t st);
 
@@ -60,10 +61,18 @@ static size_t getrf_ws_bytes(int64_t n)
     return lnb_align256(lnb_lu_perm_bytes()) + lnb_trsm_f64_ws_bytes(LU_BO, n) + 1024;
 }
 
+/* columns whose rows are permuted at a time: at most 256 MB of scratch, or a column */
+static int64_t getrs_cols(int64_t n, int64_t nrhs)
+{
+    const int64_t k = ((int64_t)1 << 25) / n;
+    return k < 1 ? 1 : k < nrhs ? k : nrhs;
+}
+
 static size_t getrs_ws_bytes(int64_t n, int64_t nrhs)
 {
+    if (n <= 0 || nrhs <= 0) return 1024;
     const size_t t = lnb_trsm_f64_ws_bytes(n, nrhs) + 1024;
-    const size_t p = lnb_align256((size_t)n * 4) + lnb_align256((size_t)n * nrhs * 8);
+    const size_t p = lnb_align256((size_t)n * 4) + lnb_align256((size_t)n * getrs_cols(n, nrhs) * 8);
     return t > p ? t : p;
 }
 
@@ -114,9 +123,12 @@ static int getrs_run(lnb_ctx *c, int64_t n, int64_t nrhs, const double *dLU, int
     if (n <= 0 || nrhs <= 0) return 0;
     lnb_arena a2 = *ar;
     int *src = lnb_arena_take(&a2, (size_t)n * 4);
-    double *T = lnb_arena_take(&a2, (size_t)n * nrhs * 8);
+    double *T = lnb_arena_take(&a2, (size_t)n * getrs_cols(n, nrhs) * 8);
     if (!src || !T) return lnb_set_error(LNB_ENOMEM, "getrs workspace");
-    CK(lnb_k_rows_permute_f64(dB, ldb, n, nrhs, n, dpiv, src, T, s), "rhs swaps");
+    if (n <= lnb_rows_permute_max())
+        CK(lnb_k_rows_permute_f64(dB, ldb, n, nrhs, n, dpiv, src, T, getrs_cols(n, nrhs), s), "rhs swaps");
+    else
+        CK(lnb_k_laswp_f64(dB, ldb, 0, n, dpiv, 0, nrhs, 0, 0, s), "rhs swaps");
     a2 = *ar;
     int e = lnb_trsm_f64_run(c, 'L', 'N', 'U', n, nrhs, 1.0, dLU, lda, dB, ldb, &a2, s, NULL);
     if (e) return e;
