@@ -13,6 +13,7 @@
 #include "common.cuh"
 #include "k_potrf.cuh"
 
+#include <cooperative_groups.h>
 #include <math.h>
 #include <stdlib.h>
 
@@ -301,26 +302,64 @@ __global__ void __launch_bounds__(128) k_trsm_rlt_f64(const double *__restrict__
 // ========================================================================
 // C = alpha op(A) op(B) + beta C, optionally restricted to a triangle of C
 // (tri = 'L' or 'U'), on DMMA: 64 x 64 CTA tiles, 4 warps of 32 x 32, BK = 16,
-// cp.async pipeline, three CTAs per SM.  Each operand is staged in the
+// cp.async pipeline, two or three CTAs per SM.  Each operand is staged in the
 // orientation its memory is contiguous in, so every copy is a 16-byte
 // cp.async along a column: op(A) = A and op(B) = B^T are stored k-major
 // (S[k][m], row stride 68), op(A) = A^T and op(B) = B m-major (S[m][k], row
 // stride 20).  Both strides spread a half-warp's fragment reads over all 32
 // banks.  beta == 0 does not read C (BLAS semantics).
-// Bound by the DMMA rate.  A thread's places in a chunk are the same for every
-// chunk, so its pointers and its rows' predicates are set once and a chunk costs
-// four copies per operand; with them computed per copy two CTAs per SM fitted and
-// the n = k = 4000 SYRK ran at 26.4 TF/s, now 31.1 (8192: 29.4, now 33.5).
+// Bound by the DMMA rate once three CTAs share every SM: there a thread's places in a
+// chunk, its pointers and its rows' predicates are set once (Loader) and a chunk costs
+// four copies per operand; with them computed per copy (load_op) only two CTAs fit
+// and the n = k = 4000 SYRK ran at 26.4 TF/s, now 31.1 (8192: 29.4, now 33.5).  With
+// fewer CTAs it is bound by one CTA's latency: four stages, load_op (its copies
+// schedule better: n = k = 1300 114 us against 133) and, where the tiles would not
+// fill the chip, K split over a cluster.
 namespace gm {
 constexpr int BM = 64, BN = 64, BK = 16, THREADS = 128;
 constexpr int LDKM = BM + 4;                  // k-major row stride (doubles)
 constexpr int LDMK = BK + 4;                  // m-major row stride
 template <bool KM> constexpr int opsize() { return KM ? BK * LDKM : BM * LDMK; }
-template <bool AKM, bool BKM> struct Cfg {
-    static constexpr int ST = 3;                                    // three CTAs in an SM's shared memory
+template <bool AKM, bool BKM, bool DEEP> struct Cfg {
+    static constexpr int ST = DEEP ? 4 : 3;                         // for two or three CTAs per SM
     static constexpr int STAGE = opsize<AKM>() + opsize<BKM>();
     static constexpr int SMEM = ST * STAGE * (int)sizeof(double);
 };
+
+// two consecutive elements src[0], src[1] (nv of them valid) -> dst[0..1]
+LNB_DEV void load2(double *dst, const double *src, int nv)
+{
+    if (nv == 2 && ((uintptr_t)src & 15) == 0) {
+        cp_async16(dst, src, true);
+    } else {
+        cp_async8(dst, nv > 0 ? src : dst, nv > 0);
+        cp_async8(dst + 1, nv > 1 ? src + 1 : dst, nv > 1);
+    }
+}
+
+// rows x BK tile of an operand whose element (r, k) is X[r + k ldx] (KM:
+// contiguous in r -> k-major smem) or X[k + r ldx] (!KM: contiguous in k ->
+// r-major smem); rows [r0, r0 + 64) of nr, k in [k0, k0 + BK) of nk
+template <bool KM>
+LNB_DEV void load_op(double *dst, const double *X, int64_t ldx, int64_t r0, int64_t nr, int64_t k0, int64_t nk,
+                     int tid)
+{
+#pragma unroll
+    for (int it = 0; it < (BM * BK / 2) / THREADS; ++it) {
+        const int idx = tid + it * THREADS;
+        if (KM) {
+            const int kk = idx / (BM / 2), rr = (idx % (BM / 2)) * 2;
+            const int64_t r = r0 + rr, k = k0 + kk;
+            const int nv = k < nk ? (int)(r + 1 < nr ? 2 : (r < nr ? 1 : 0)) : 0;
+            load2(dst + kk * LDKM + rr, X + (nv ? r + k * ldx : 0), nv);
+        } else {
+            const int rr = idx / (BK / 2), kk = (idx % (BK / 2)) * 2;
+            const int64_t r = r0 + rr, k = k0 + kk;
+            const int nv = r < nr ? (int)(k + 1 < nk ? 2 : (k < nk ? 1 : 0)) : 0;
+            load2(dst + rr * LDMK + kk, X + (nv ? k + r * ldx : 0), nv);
+        }
+    }
+}
 
 // One thread's share of an operand's chunks: four places, 16 bytes each.  Element
 // (r, k) of the operand is X[r + k ldx] (KM) or X[k + r ldx]; rows [r0, r0 + 64) of
@@ -389,27 +428,49 @@ struct Loader {
 };
 
 // AKM: op(A) = A (k-major staging); BKM: op(B) = B^T (k-major staging)
-template <bool AKM, bool BKM>
-__global__ void __launch_bounds__(THREADS, 3) k_gemm_dmma(int64_t M, int64_t N, int64_t K, double alpha,
+// SPLIT: the CTAs of a cluster (along z) take K in consecutive parts of one tile and each
+// finishes 1/S of its elements, adding the parts in their order over DSMEM
+template <bool AKM, bool BKM, bool DEEP, bool SPLIT>
+__global__ void __launch_bounds__(THREADS, DEEP ? 2 : 3) k_gemm_dmma(int64_t M, int64_t N, int64_t K, double alpha,
                                                           const double *__restrict__ A, int64_t lda,
                                                           const double *__restrict__ B, int64_t ldb, double beta,
                                                           double *C, int64_t ldc, char tri)
 {
-    using Cf = Cfg<AKM, BKM>;
+    using Cf = Cfg<AKM, BKM, DEEP>;
     constexpr int ST = Cf::ST;
-    const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
-    if (tri == 'L' && m0 + BM <= n0) return;
-    if (tri == 'U' && n0 + BN <= m0) return;
+    int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
+    if (tri) {                                     // the triangle's tiles alone, by rows of the lower one
+        const int64_t id = blockIdx.x;
+        int64_t i = (int64_t)((sqrt(8.0 * (double)id + 1.0) - 1.0) * 0.5);
+        while (i * (i + 1) / 2 > id) --i;
+        while ((i + 1) * (i + 2) / 2 <= id) ++i;
+        const int64_t j = id - i * (i + 1) / 2;
+        m0 = (tri == 'L' ? i : j) * BM;
+        n0 = (tri == 'L' ? j : i) * BN;
+    }
     extern __shared__ __align__(16) double gsm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wm = warp >> 1, wn = warp & 1, g = lane >> 2, t = lane & 3;
-    const int ktiles = (int)((K + BK - 1) / BK);
+    int ktiles = (int)((K + BK - 1) / BK);
+    const int S = SPLIT ? (int)gridDim.z : 1, part = SPLIT ? (int)blockIdx.z : 0;
+    if (SPLIT) {
+        const int k0 = (int)((int64_t)ktiles * part / S), k1 = (int)((int64_t)ktiles * (part + 1) / S);
+        A += AKM ? (int64_t)k0 * BK * lda : k0 * BK;
+        B += BKM ? (int64_t)k0 * BK * ldb : k0 * BK;
+        K = (K < (int64_t)k1 * BK ? K : (int64_t)k1 * BK) - (int64_t)k0 * BK;
+        ktiles = k1 - k0;
+    }
     Loader<AKM> la(A, lda, m0, M, K);
     Loader<BKM> lb(B, ldb, n0, N, K);
     const uint32_t s0 = smem_u32(gsm);
     auto stage = [&](int s, int kt) {
-        la.load(s0 + s * (Cf::STAGE * 8), kt * BK);
-        lb.load(s0 + s * (Cf::STAGE * 8) + opsize<AKM>() * 8, kt * BK);
+        if constexpr (DEEP) {
+            load_op<AKM>(gsm + s * Cf::STAGE, A, lda, m0, M, (int64_t)kt * BK, K, tid);
+            load_op<BKM>(gsm + s * Cf::STAGE + opsize<AKM>(), B, ldb, n0, N, (int64_t)kt * BK, K, tid);
+        } else {
+            la.load(s0 + s * (Cf::STAGE * 8), kt * BK);
+            lb.load(s0 + s * (Cf::STAGE * 8) + opsize<AKM>() * 8, kt * BK);
+        }
     };
     double acc[2][4][4];
 #pragma unroll
@@ -454,6 +515,40 @@ __global__ void __launch_bounds__(THREADS, 3) k_gemm_dmma(int64_t M, int64_t N, 
         }
     }
     cp_async_wait<0>();
+    if constexpr (SPLIT) {
+        cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        __syncthreads();                           // the ring is read
+        double *red = gsm;                         // [element of a thread][thread]
+#pragma unroll
+        for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) red[(mi * 16 + ni * 4 + q) * THREADS + tid] = acc[mi][ni][q];
+        cl.sync();
+        for (int e0 = part * (32 / S); e0 < (part + 1) * (32 / S); e0 += 4) {
+            const int mi = e0 >> 4, ni = (e0 >> 2) & 3;
+            const int64_t r0 = m0 + wm * 32 + mi * 16 + g, c0 = n0 + wn * 32 + ni * 8 + 2 * t;
+            double v[4] = {0.0, 0.0, 0.0, 0.0}, cv[4];
+            for (int z = 0; z < S; ++z) {
+                const double *rz = cl.map_shared_rank(red, z) + e0 * THREADS + tid;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] += rz[q * THREADS];
+            }
+            auto keep = [&](int q) {
+                const int64_t r = r0 + (q >> 1) * 8, c = c0 + (q & 1);
+                return r < M && c < N && !(tri == 'L' && r < c) && !(tri == 'U' && r > c);
+            };
+            double *cp = C + r0 + c0 * ldc;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                cv[q] = beta != 0.0 && keep(q) ? beta * cp[(q >> 1) * 8 + (q & 1) * ldc] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (keep(q)) cp[(q >> 1) * 8 + (q & 1) * ldc] = __dadd_rn(cv[q], __dmul_rn(alpha, v[q]));
+        }
+        cl.sync();                                 // no CTA leaves while its part may be read
+    } else {
     // sixteen loads of C in flight: through one pointer the compiler would finish
     // each read-modify-write before the next
 #pragma unroll
@@ -476,7 +571,22 @@ __global__ void __launch_bounds__(THREADS, 3) k_gemm_dmma(int64_t M, int64_t N, 
             for (int q = 0; q < 4; ++q)
                 if (keep(ni, q)) cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] = __dadd_rn(cv[ni][q], __dmul_rn(alpha, acc[mi][ni][q]));
     }
+    }
 }
+// Parts K is split into: as many (8, 4 or 2) as keep all CTAs resident, three on each of
+// the 148 SMs, with 128 or more of K each.  SYRK in one part / split, start to end:
+// n = 220, k = 5035 (10 tiles) 336 us / 46 in eight; n = k = 500 (36) 45 / 19 in four;
+// n = k = 1000 (136) 91 / 52 in two.
+inline int splits(int64_t tiles, int64_t K)
+{
+    const int64_t kt = (K + BK - 1) / BK;
+    for (int S = 8; S > 1; S /= 2)
+        if (tiles * S <= 3 * 148 && kt / S >= 8) return S;
+    return 1;
+}
+// Four stages and two CTAs per SM where three CTAs per SM would not fill the chip, or would
+// leave a nearly empty second wave (n = 1900, k = 3000, 465 tiles: 482 us, with three 596).
+inline bool deep(int64_t ctas) { return ctas <= 2 * 148 || (ctas > 3 * 148 && ctas <= 4 * 148); }
 }  // namespace gm
 
 }  // namespace lnb
@@ -549,19 +659,49 @@ extern "C" int lnb_k_syrk_lower_f64(const double *P, int64_t ldp, double *C, int
     }
 }
 
-template <bool AKM, bool BKM>
-static void launch_gemm(int64_t m, int64_t n, int64_t k, double alpha, const double *A, int64_t lda,
-                        const double *B, int64_t ldb, double beta, double *C, int64_t ldc, char tri, lnb_stream_t s)
+template <bool AKM, bool BKM, bool DEEP, bool SPLIT>
+static int launch_gemm_as(dim3 grid, int64_t m, int64_t n, int64_t k, double alpha, const double *A, int64_t lda,
+                          const double *B, int64_t ldb, double beta, double *C, int64_t ldc, char tri, lnb_stream_t s)
 {
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(gm::k_gemm_dmma<AKM, BKM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             gm::Cfg<AKM, BKM>::SMEM);
-        attr = true;
-    }
-    dim3 grid((unsigned)((n + gm::BN - 1) / gm::BN), (unsigned)((m + gm::BM - 1) / gm::BM));
-    gm::k_gemm_dmma<AKM, BKM><<<grid, gm::THREADS, gm::Cfg<AKM, BKM>::SMEM, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
-                                                                  tri);
+    constexpr int SMEM = gm::Cfg<AKM, BKM, DEEP>::SMEM;
+    static_assert(SMEM >= 32 * gm::THREADS * (int)sizeof(double), "a part fits the ring");
+    auto kern = gm::k_gemm_dmma<AKM, BKM, DEEP, SPLIT>;
+    /* The shared memory asked for keeps the CTAs spread out, one or two per SM: where three
+       fit, some SMs got three and others none (n = k = 1300: 166 us, so 113).  Clusters of one CTA per
+       SM do not fill every SM (144 CTAs by fours took two waves), so only up to 96 CTAs. */
+    const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
+    const int smem = !DEEP ? SMEM : ctas <= (SPLIT ? 96 : 148) ? 116 * 1024 : SMEM > 80 * 1024 ? SMEM : 80 * 1024;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(gm::THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = grid.z;
+    cfg.attrs = at;
+    cfg.numAttrs = SPLIT ? 1 : 0;
+    return (int)cudaLaunchKernelEx(&cfg, kern, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri);
+}
+
+template <bool AKM, bool BKM>
+static int launch_gemm(int64_t m, int64_t n, int64_t k, double alpha, const double *A, int64_t lda,
+                       const double *B, int64_t ldb, double beta, double *C, int64_t ldc, char tri, lnb_stream_t s)
+{
+    const int64_t tm = (m + gm::BM - 1) / gm::BM, tn = (n + gm::BN - 1) / gm::BN;
+    const int64_t tiles = tri ? tn * (tn + 1) / 2 : tm * tn;
+    const int S = gm::splits(tiles, k);
+    const bool deep = gm::deep(tiles * S);
+    const dim3 grid((unsigned)(tri ? tiles : tn), (unsigned)(tri ? 1 : tm), (unsigned)S);
+    if (S > 1)
+        return deep ? launch_gemm_as<AKM, BKM, true, true>(grid, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s)
+                    : launch_gemm_as<AKM, BKM, false, true>(grid, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s);
+    return deep ? launch_gemm_as<AKM, BKM, true, false>(grid, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s)
+                : launch_gemm_as<AKM, BKM, false, false>(grid, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s);
 }
 
 extern "C" int lnb_k_gemm_tri_f64(char ta, char tb, int64_t m, int64_t n, int64_t k, double alpha,
@@ -570,11 +710,12 @@ extern "C" int lnb_k_gemm_tri_f64(char ta, char tb, int64_t m, int64_t n, int64_
 {
     if (m <= 0 || n <= 0) return 0;
     const bool akm = ta == 'N', bkm = tb == 'T';
-    if (akm && bkm) launch_gemm<true, true>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s);
-    else if (akm) launch_gemm<true, false>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s);
-    else if (bkm) launch_gemm<false, true>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s);
-    else launch_gemm<false, false>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s);
+    int e;
+    if (akm && bkm) e = launch_gemm<true, true>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s);
+    else if (akm) e = launch_gemm<true, false>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s);
+    else if (bkm) e = launch_gemm<false, true>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s);
+    else e = launch_gemm<false, false>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri, s);
     lnb_prof_count(1);
-    return (int)cudaGetLastError();
+    return e ? e : (int)cudaGetLastError();
 }
 
