@@ -216,11 +216,11 @@ LNB_EXPORT int lnb_dchol_noalloc_dev(int n, int b, double *dA, int lda, int *inf
  *     fused DMMA trailing updates behind them): best for large n.
  *   LNB_SCHED_DAG: one persistent launch that walks the tile task DAG on the
  *     device (64 x 64 tiles handed out by an atomic ticket in priority order,
- *     dependencies tracked by per-tile flags, every wait bounded): best where
+ *     dependencies tracked by progress counters, every wait bounded): best where
  *     the critical path dominates.  The tile size b only shapes the stream
  *     schedule; the DAG uses its own 64-wide tiles (the factor is the same up
  *     to rounding).
- *   LNB_SCHED_AUTO (default): the device DAG for n <= 4096, streams above. */
+ *   LNB_SCHED_AUTO (default): the device DAG for n <= 16384, streams above. */
 #define LNB_SCHED_AUTO     0
 #define LNB_SCHED_STREAMS  1
 #define LNB_SCHED_DAG      2
