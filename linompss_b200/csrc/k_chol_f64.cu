@@ -549,28 +549,30 @@ __global__ void __launch_bounds__(THREADS, DEEP ? 2 : 3) k_gemm_dmma(int64_t M, 
         }
         cl.sync();                                 // no CTA leaves while its part may be read
     } else {
-    // sixteen loads of C in flight: through one pointer the compiler would finish
-    // each read-modify-write before the next
+        // sixteen loads of C in flight: through one pointer the compiler would finish
+        // each read-modify-write before the next
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi) {
-        const int64_t r0 = m0 + wm * 32 + mi * 16 + g, c0 = n0 + wn * 32 + 2 * t;
-        double *cp = C + r0 + c0 * ldc;
-        auto keep = [&](int ni, int q) {
-            const int64_t r = r0 + (q >> 1) * 8, c = c0 + ni * 8 + (q & 1);
-            return r < M && c < N && !(tri == 'L' && r < c) && !(tri == 'U' && r > c);
-        };
-        double cv[4][4];
+        for (int mi = 0; mi < 2; ++mi) {
+            const int64_t r0 = m0 + wm * 32 + mi * 16 + g, c0 = n0 + wn * 32 + 2 * t;
+            double *cp = C + r0 + c0 * ldc;
+            auto keep = [&](int ni, int q) {
+                const int64_t r = r0 + (q >> 1) * 8, c = c0 + ni * 8 + (q & 1);
+                return r < M && c < N && !(tri == 'L' && r < c) && !(tri == 'U' && r > c);
+            };
+            double cv[4][4];
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+            for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                cv[ni][q] = beta != 0.0 && keep(ni, q) ? beta * cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] : 0.0;
+                for (int q = 0; q < 4; ++q)
+                    cv[ni][q] = beta != 0.0 && keep(ni, q) ? beta * cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] : 0.0;
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+            for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (keep(ni, q)) cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] = __dadd_rn(cv[ni][q], __dmul_rn(alpha, acc[mi][ni][q]));
-    }
+                for (int q = 0; q < 4; ++q)
+                    if (keep(ni, q))
+                        cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] =
+                            __dadd_rn(cv[ni][q], __dmul_rn(alpha, acc[mi][ni][q]));
+        }
     }
 }
 // Parts K is split into: as many (8, 4 or 2) as keep all CTAs resident, three on each of
