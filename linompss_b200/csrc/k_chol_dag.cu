@@ -129,17 +129,24 @@ LNB_DEV double pivot_rsqrt(double d)
 // inv(L_pp)^T, Xs[c * LDX + r], comes out of the same column steps applied to
 // eight identity rows.  A warp holds the eight pivot rows in lanes 0-7 and 48 of
 // the other rows (the identity rows first) in the other lanes, two per lane;
-// panels 0 and 1 take two warps, which repeat the pivot rows and so need not
-// wait for each other.  Every lane tracks the pivots (dd): it takes the pivot
-// rows' entries of the column by shuffle before they are scaled, so the chain
-// per column is 1/sqrt -> multiply -> fma, and the shuffles and the rows'
-// updates run beside it.  The fast form takes every pivot as a normal positive
+// panels 0 and 1 take two warps, which both work on the pivot rows: they meet at
+// a barrier between the loads and the first store, because warp 0 stores the
+// finished pivot rows where warp 1 loads them.  Every lane tracks the pivots
+// (dd): it takes the pivot rows' entries of the column by shuffle before they are
+// scaled, so the chain per column is 1/sqrt -> multiply -> fma, and the shuffles
+// and the rows' updates run beside it.  The fast form takes every pivot as a normal positive
 // number and looks at them after the last column (a branch or a select per
 // column costs 100 - 270 of its 760 cycles); where one is not, it stores
 // nothing and the other form repeats the panel.  Returns the tile column of the
 // first non-positive pivot (its column and those after it keep their values),
 // 64 if there is none, or -1 (fast form) to ask for the repetition.
 LNB_DEV int panel_warps(int p) { return p < 2 ? 2 : 1; }
+// every panel warp has loaded its rows (both see the same pivots, so both repeat a panel or
+// neither does)
+LNB_DEV void panel_loaded(int p)
+{
+    if (panel_warps(p) == 2) asm volatile("bar.sync 2, 64;" ::: "memory");
+}
 template <bool FAST>
 LNB_DEV int warp_panel8(double *Sc, double *Xs, int p, int w)
 {
@@ -155,6 +162,7 @@ LNB_DEV int warp_panel8(double *Sc, double *Xs, int p, int w)
         b[k] = col1[k * LDK];
         if (!real0) a[k] = ident && k == i0 ? 1.0 : 0.0;
     }
+    panel_loaded(p);
 #pragma unroll
     for (int k = 0; k < PW; ++k) dd[k] = __shfl_sync(0xffffffffu, a[k], k);
     int fail = TS;

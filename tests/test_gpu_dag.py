@@ -143,3 +143,24 @@ def test_dag_wait_runs_out_and_context_stays_usable(lnb):
     A = A0.copy(order="F")
     assert lnb.ompss_dchol_rl(n, 64, 64, A, n) == 0
     np.testing.assert_allclose(np.tril(A), np.linalg.cholesky(A0), rtol=0, atol=1e-11)
+
+
+def test_dag_factor_repeats_bit_for_bit(lnb, cuda):
+    """Every sum of the walk has a fixed order, so a factor is the same in every run, also beside other work.  (Two
+    warps share a diagonal tile's first panels: a load of a pivot row after its store would show here as another
+    factor.)"""
+    import torch
+    n = 1000
+    A = torch.tensor(np.ascontiguousarray(O.spd_covariance(n, 0.5, seed=1)), device=cuda)
+    other, X = torch.cuda.Stream(), torch.randn(2048, 2048, device=cuda)
+    first = None
+    for rep in range(100):
+        At = A.clone()
+        with torch.cuda.stream(other):
+            X = torch.tanh(X @ X)
+        lnb.dchol_dev(At, n, 256)
+        if first is None:
+            first = At
+            L = torch.linalg.cholesky(A)
+            assert float((torch.triu(At) - L.T).abs().max()) <= 64 * n * EPS * float(L.abs().max())
+        assert torch.equal(At, first), rep
