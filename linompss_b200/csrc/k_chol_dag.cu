@@ -134,8 +134,8 @@ LNB_DEV double pivot_rsqrt(double d)
 // finished pivot rows where warp 1 loads them.  Every lane tracks the pivots
 // (dd): it takes the pivot rows' entries of the column by shuffle before they are
 // scaled, so the chain per column is 1/sqrt -> multiply -> fma, and the shuffles
-// and the rows' updates run beside it.  The fast form takes every pivot as a normal positive
-// number and looks at them after the last column (a branch or a select per
+// and the rows' updates run beside it.  The fast form takes every pivot as a finite
+// normal positive number and looks at them after the last column (a branch or a select per
 // column costs 100 - 270 of its 760 cycles); where one is not, it stores
 // nothing and the other form repeats the panel.  Returns the tile column of the
 // first non-positive pivot (its column and those after it keep their values),
@@ -193,7 +193,8 @@ LNB_DEV int warp_panel8(double *Sc, double *Xs, int p, int w)
         double lo = dd[0];                                   // a NaN fails the comparison below
 #pragma unroll
         for (int c = 1; c < PW; ++c) lo = dd[c] < lo || !(dd[c] == dd[c]) ? dd[c] : lo;
-        if (!(lo >= 2.2250738585072014e-308)) return -1;     // warp-uniform: dd is broadcast
+        // an infinite pivot makes the ones after it NaN; the last has none after it
+        if (!(lo >= 2.2250738585072014e-308 && dd[PW - 1] <= 1.7976931348623157e308)) return -1;   // warp-uniform
     }
     if (ident) {
 #pragma unroll

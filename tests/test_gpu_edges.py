@@ -142,6 +142,22 @@ def test_chol_extreme_scale(lnb, sched, exp):
     assert (np.abs(L @ L.T - As) - extra).max() <= 4 * (n + 64) * U * d.max() ** 2
 
 
+@pytest.mark.parametrize("pos", [0, 6, 7, 15, 63, 71, 149])
+def test_chol_infinite_pivot(lnb, pos):
+    """1/sqrt(inf) = 0: the column below an infinite pivot is zero wherever it stands in its panel, so the rest of the
+    factor is that of the matrix without this row and column"""
+    lnb.set_chol_schedule(lnb.SCHED_DAG)
+    n = 150
+    A0 = O.spd_covariance(n, 0.5, seed=4)
+    A = A0.copy(order="F")
+    A[pos, pos] = np.inf
+    assert lnb.ompss_dchol_rl(n, 64, 64, A, n) == 0
+    L = np.tril(A)
+    np.testing.assert_array_equal(L[pos + 1:, pos], 0.0)
+    keep = np.arange(n) != pos
+    check_chol(A0[np.ix_(keep, keep)], L[np.ix_(keep, keep)], n)
+
+
 @pytest.mark.parametrize("sched", ["SCHED_DAG", "SCHED_STREAMS"])
 @pytest.mark.parametrize("pos", [0, 1, 31, 32, 63, 64, 95, 127, 128, 199])
 def test_chol_failed_pivot(lnb, sched, pos):
