@@ -111,11 +111,15 @@ LNB_DEV bool mma_sync_and(bool pred)
     return r != 0;
 }
 
-// 1/sqrt(d) for a normal d > 0: the approximate instruction (relative error
-// 2^-20 measured) and one third-order step of the iteration
-// y' = y (1 + h/2 + 3 h^2/8), h = 1 - d y^2 (Householder's method for y^-2 = d),
-// which leaves the last rounding (1.4e-16 measured).  No branch: rsqrt()'s
-// special-case branch would fence the column's other work off its latency.
+// 1/sqrt(d) for a normal d > 0: the approximate instruction, then one step of
+// Householder's iteration of third order (A. S. Householder, The Numerical
+// Treatment of a Single Nonlinear Equation, 1970) for y^-2 = d:
+// y' = y (1 + h/2 + 3 h^2/8), h = 1 - d y^2, whose next term is 5 h^3/16.  With the
+// instruction's error below 2^-20 (|h| < 2^-19) that term is 0.02 u; the roundings of
+// h and of the last sum are 1.5 u (u = 2^-53).  tests/test_gpu_edges.py holds the
+// result to 1.6 u of the exact value and compares it with rsqrt().  Calling rsqrt()
+// here instead: n = 200 with one solve 135 us against 125, n = 5003 1.928 ms against
+// 1.896.
 LNB_DEV double pivot_rsqrt(double d)
 {
     double y;

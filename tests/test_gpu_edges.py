@@ -142,6 +142,35 @@ def test_chol_extreme_scale(lnb, sched, exp):
     assert (np.abs(L @ L.T - As) - extra).max() <= 4 * (n + 64) * U * d.max() ** 2
 
 
+@pytest.mark.parametrize("lo,hi", [(-1022, 1023), (-3, 3), (0, 0)])
+def test_chol_reciprocal_root(lnb, cuda, lo, hi):
+    """1/sqrt of a pivot d = 2^e m, e in [lo, hi]: [[d, 1], [1, c]] blocks leave 1 * (1/sqrt(d)) in L_21, exactly what
+    the factor multiplies its columns by.  The walk's own iteration loses 1.5 u to its two roundings and 0.02 u to the
+    series: at most 1.6 u off the exact value, and 3.6 u off CUDA's rsqrt (1 ulp, up to 2 u)."""
+    import torch
+    lnb.set_chol_schedule(lnb.SCHED_DAG)
+    n, rng = 4096, np.random.default_rng(hi)
+    for _ in range(3):
+        d = np.ldexp(rng.uniform(1, 2, n // 2), rng.integers(lo, hi + 1, n // 2))
+        d[:4] = np.ldexp([1.0, 1.0, 2 - 2.0 ** -52, 2 - 2.0 ** -52], [lo, hi, lo, hi])
+        diag = np.empty(n)
+        diag[::2] = d
+        diag[1::2] = np.maximum(2 / d, 1.0)                     # the second pivot, c - 1/d, is normal and positive
+        At = torch.diag(torch.tensor(diag, device=cuda))
+        i = torch.arange(0, n, 2, device=cuda)
+        At[i, i + 1] = 1.0                                      # column-major: A[i + 1, i]
+        info = torch.full((1,), -9, dtype=torch.int32, device=cuda)
+        lnb.dchol_dev(At, n, 256, info=info)
+        assert int(info.item()) == 0
+        got = At[i, i + 1].cpu().numpy()
+        exact = 1 / np.sqrt(d.astype(np.longdouble))
+        assert np.abs(got / exact - 1).max() <= 1.6 * U
+        cuda_rsqrt = torch.rsqrt(torch.tensor(d, device=cuda)).cpu().numpy()
+        assert np.abs(got / cuda_rsqrt.astype(np.longdouble) - 1).max() <= 3.6 * U
+        root = At[i, i].cpu().numpy()                           # d * (1/sqrt(d)): one more rounding
+        assert np.abs(root * exact - 1).max() <= 2.7 * U
+
+
 @pytest.mark.parametrize("pos", [0, 6, 7, 15, 63, 71, 149])
 def test_chol_infinite_pivot(lnb, pos):
     """1/sqrt(inf) = 0: the column below an infinite pivot is zero wherever it stands in its panel, so the rest of the
