@@ -105,16 +105,6 @@ LNB_DEV void warp_best(unsigned long long &key, int &idx)
     key = (unsigned long long)mh << 32 | ml;
 }
 
-// 1/x for |x| in [1e-280, 1e280]: the approximate instruction (relative error
-// 2^-20) and one third-order step y' = y (1 + e + e^2), e = 1 - x y
-LNB_DEV double pivot_rcp(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-
 // The panel.  Bound by latency: each column is a pivot search over all rows, a row
 // broadcast and a rank-1 step, one after another.  A thread holds whole rows of the
 // panel in registers (moved down one place per column, so indexes stay constant),
@@ -224,11 +214,15 @@ __global__ void __launch_bounds__(PT, 1) k_lu_panel(double *A, int64_t lda, int6
             krow = (const double *)S.ckrow[b];
         }
         const double pv = prow[0];
-        // l = a / pv: the quotient by the reciprocal, corrected by its remainder
-        // (|a| <= |pv|); a zero pivot divides nothing, as in dgetf2
+        // l = a / pv (|a| <= |pv|): one division per column for 1 / pv, then the product
+        // with it corrected by its remainder, which rounds as the division does
+        // (P. W. Markstein, Computation of Elementary Functions on the IBM RISC
+        // System/6000 Processor, IBM J. Res. Dev. 34, 1990); plain divisions where
+        // 1 / pv or the remainder may leave the range.  n = 1500: 3.40 ms, with a
+        // division per element 3.65.  A zero pivot divides nothing, as in dgetf2.
         const double apv = fabs(pv);
         const bool plain = apv >= 1e-280 && apv <= 1e280;
-        const double rp = pivot_rcp(pv);
+        const double rp = 1.0 / pv;
         // 3. row p takes the old row k
         if (p >= base && p < base + PT * RPT && ((p - base) % PT) >> 5 == warp) {
 #pragma unroll

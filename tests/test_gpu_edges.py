@@ -261,6 +261,36 @@ def test_getrf_edges(lnb, cuda, m, n, pad, off):
     check_lu(A0, got[:, :m].T, piv)
 
 
+@pytest.mark.parametrize("rows", [512, 3000, 20000])
+def test_getrf_multipliers(lnb, cuda, rows):
+    """L's columns are the quotients a / pivot.  The panel forms them as a (1 / pivot) with the remainder put right
+    (Markstein's theorem): the division's own bits, checked against numpy's division, wherever the remainder is exact
+    (|a| >= 2^-968: its last bit is then at or above 2^-1074) and the quotient is normal; elsewhere within the last
+    place.  Pivots on both sides of the range in which it does so, 1e-280 and 1e280."""
+    import torch
+    rng = np.random.default_rng(rows)
+    tiny = np.finfo(np.float64).tiny
+    for e in [0, 3, -700, 700, -929, -930, -931, 929, 930, 931, -1000, 1000, -1021, 1023]:
+        pv = np.ldexp(rng.uniform(1, 2), e) * rng.choice([-1.0, 1.0])
+        a = pv * rng.uniform(-1, 1, rows)
+        a[1::2] = np.ldexp(a[1::2], rng.integers(-200, 1, a[1::2].size))
+        a[3:6] = [0.0, np.nextafter(pv, 0), tiny * np.sign(pv)]
+        a[7] = pv
+        A0 = a[:, None].copy()
+        At, _ = dev(cuda, A0)
+        ipiv = torch.zeros(1, dtype=torch.int32, device=cuda)
+        lnb.dgetrf_dev(At, rows, 1, ipiv)
+        assert int(ipiv.item()) == 8
+        got = At.cpu().numpy()[0]
+        a[[0, 7]] = a[[7, 0]]
+        with np.errstate(under="ignore"):
+            q = a[1:] / pv
+        assert got[0] == pv
+        exact = (np.abs(a[1:]) >= 2.0 ** -968) & (np.abs(q) >= tiny) | (a[1:] == 0)
+        np.testing.assert_array_equal(got[1:][exact], q[exact])
+        assert (np.abs(got[1:] - q) <= np.spacing(np.abs(q))).all(), e
+
+
 @pytest.mark.parametrize("n,nrhs,pad", [(1, 1, 0), (33, 1, 1), (1000, 3, 1), (1025, 17, 0), (1000, 40000, 0)])
 def test_getrs_edges(lnb, cuda, n, nrhs, pad):
     """row exchanges of the right-hand sides, in one slice of scratch and in several (n nrhs > 32 Mi)"""
