@@ -351,6 +351,26 @@ def test_syrk_edges(lnb, cuda, uplo, trans, n, k, pad, off):
     assert (err <= 2 * (k + 4) * U * (0.5 * np.abs(a) @ np.abs(a).T + 2 * np.abs(Cm))).all()
 
 
+# one term per element, so the sum is exact up to its one rounding, and the last step is visible: alpha P is not
+# rounded before beta C joins.  m, n, k reach one CTA's form, K split over a cluster, and three CTAs per SM
+@pytest.mark.parametrize("m,n,k", [(65, 63, 1), (200, 100, 2100), (1500, 1400, 3)])
+@pytest.mark.parametrize("beta", [0.0, 0.7])
+def test_gemm_epilogue_is_fused(lnb, cuda, m, n, k, beta):
+    import torch
+    from fractions import Fraction
+    rng = np.random.default_rng(m)
+    A, B = np.zeros((m, k)), np.zeros((k, n))
+    A[:, k // 2], B[k // 2] = rng.standard_normal(m), rng.standard_normal(n)
+    Cm = rng.standard_normal((m, n))
+    alpha = 1.1
+    (At, _), (Bt, _), (Ct, _) = dev(cuda, A), dev(cuda, B), dev(cuda, Cm)
+    lnb.dgemm_dev("N", "N", m, n, k, alpha, At, Bt, beta, Ct)
+    got = Ct.cpu().numpy().T
+    for r, c in zip(rng.integers(0, m, 2000), rng.integers(0, n, 2000)):
+        p = A[r, k // 2] * B[k // 2, c]
+        assert got[r, c] == float(Fraction(alpha) * Fraction(p) + Fraction(beta * Cm[r, c])), (r, c)
+
+
 # ---------------------------------------------------------------- dense CG in one launch
 @pytest.mark.parametrize("n,steps", [(1, 3), (2, 1), (31, 4), (33, 0), (64, 5), (1000, 6), (1501, 3)])
 def test_dcg_edges(lnb, n, steps):
