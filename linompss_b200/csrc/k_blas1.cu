@@ -420,7 +420,9 @@ extern "C" int lnb_k_dcg_f64(int64_t n, const double *A, int64_t lda, const doub
     cudaError_t e = cudaMemsetAsync(sync, 0, 64 * sizeof(int), (cudaStream_t)s);
     if (e != cudaSuccess) return (int)e;
     const int smem = (int)(2 * n * sizeof(double));
-    e = cudaFuncSetAttribute(k_dcg, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    /* the largest of any call, as several host threads may set it */
+    e = cudaFuncSetAttribute(k_dcg, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(2 * lnb_dcg_max_n() * sizeof(double)));
     if (e != cudaSuccess) return (int)e;
     const int64_t tiles = rgs * a.cs;
     const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);

@@ -672,8 +672,12 @@ static int launch_gemm_as(dim3 grid, int64_t m, int64_t n, int64_t k, double alp
        fit, some SMs got three and others none (n = k = 1300: 166 us, so 113).  Clusters of one CTA per
        SM do not fill every SM (144 CTAs by fours took two waves), so only up to 96 CTAs. */
     const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
-    const int smem = !DEEP ? SMEM : ctas <= (SPLIT ? 96 : 148) ? 116 * 1024 : SMEM > 80 * 1024 ? SMEM : 80 * 1024;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    constexpr int ONE = 116 * 1024, TWO = SMEM > 80 * 1024 ? SMEM : 80 * 1024;
+    const int smem = !DEEP ? SMEM : ctas <= (SPLIT ? 96 : 148) ? ONE : TWO;
+    /* always the most that any launch of this kernel asks for: calls of several host
+       threads may stand between here and the launch */
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               !DEEP ? SMEM : ONE > TWO ? ONE : TWO);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;

@@ -629,7 +629,8 @@ extern "C" int lnb_k_rows_permute_f64(double *B, int64_t ldb, int64_t n, int64_t
     if (n <= 0 || nrhs <= 0 || k1 <= 0) return 0;
     if (n > lnb_rows_permute_max()) return (int)cudaErrorInvalidValue;
     const int smem = (int)((n + 3) & ~3ll) * 4 + 32 * (int)sizeof(Chunk);
-    cudaError_t e = cudaFuncSetAttribute(k_piv_compose, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    /* the largest of any call, as several host threads may set it */
+    cudaError_t e = cudaFuncSetAttribute(k_piv_compose, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return (int)e;
     k_piv_compose<<<1, 1024, smem, (cudaStream_t)s>>>((int)n, (int)k1, piv, src);
     lnb_prof_count(1);

@@ -371,6 +371,41 @@ def test_gemm_epilogue_is_fused(lnb, cuda, m, n, k, beta):
         assert got[r, c] == float(Fraction(alpha) * Fraction(p) + Fraction(beta * Cm[r, c])), (r, c)
 
 
+def test_gemm_from_two_threads(lnb, cuda):
+    """products use no workspace, so calls of several host threads may meet: neither may undo what the other's launch
+    needs (the two orders here take different amounts of shared memory)"""
+    import ctypes as C
+    import torch
+    errors, k = [], 8
+    call = C.CDLL(lnb.LIB_PATH).lnb_dgemm_dev                  # the bare function: as little Python per call as can be
+
+    def work(n):
+        torch.cuda.set_device(cuda)
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            A, B = (torch.randn(n, k, dtype=torch.float64, device=cuda) for _ in range(2))
+            Ct = torch.zeros(n, n, dtype=torch.float64, device=cuda)
+        args = (C.c_char(b"T"), C.c_char(b"N"), C.c_int(n), C.c_int(n), C.c_int(k), C.c_double(1.0),
+                C.c_void_p(A.data_ptr()), C.c_int(k), C.c_void_p(B.data_ptr()), C.c_int(k), C.c_double(0.0),
+                C.c_void_p(Ct.data_ptr()), C.c_int(n), C.c_void_p(s.cuda_stream))
+        rcs = set()
+        for i in range(10000):
+            rcs.add(call(*args))
+            if i % 10 == 0:
+                s.synchronize()
+        s.synchronize()
+        ok = bool(((Ct.T - A @ B.T).abs() <= 2 * (k + 4) * U * (A.abs() @ B.abs().T)).all())
+        if rcs != {0} or not ok:
+            errors.append((n, rcs, ok))
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in (500, 1000)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+
+
 # ---------------------------------------------------------------- dense CG in one launch
 @pytest.mark.parametrize("n,steps", [(1, 3), (2, 1), (31, 4), (33, 0), (64, 5), (1000, 6), (1501, 3)])
 def test_dcg_edges(lnb, n, steps):
