@@ -267,5 +267,8 @@ int lnb_dgetrs_dev(int n, int nrhs, const double *dLU, int lda, const int *dipiv
     void *ws = lnb_ws(c, getrs_ws_bytes(n, nrhs) + 1024);
     if (!ws) return LNB_ENOMEM;
     lnb_arena ar = {(char *)ws, 0, c->ws_size};
-    return getrs_run(c, n, nrhs, dLU, lda, dipiv, dB, ldb, &ar, (cudaStream_t)stream);
+    cudaStream_t s = (cudaStream_t)stream;
+    /* the solves' waits give up at a recorded timeout: an earlier call's must not stand */
+    CK(cudaMemsetAsync(c->st, 0, sizeof(lnb_status_t), s), "status reset");
+    return getrs_run(c, n, nrhs, dLU, lda, dipiv, dB, ldb, &ar, s);
 }

@@ -312,6 +312,28 @@ def test_getrs_edges(lnb, cuda, n, nrhs, pad):
     assert float(R.max() / scale) <= 12 * (n + 64) * U        # three such bounds: factor and two solves
 
 
+@pytest.mark.parametrize("n,nrhs", [(1000, 3), (4096, 300), (1024, 8192)])
+def test_getrs_after_a_timeout(lnb, cuda, n, nrhs):
+    """a timeout that an earlier call left in the status word is not this call's (its waits look at that word once
+    they have polled for a while: many columns)"""
+    import ctypes
+    import torch
+    lib = lnb.lib()
+    lib.lnb_selftest_wait_timeout.argtypes = [ctypes.c_longlong]
+    g = torch.Generator(cuda).manual_seed(n)
+    A = torch.randn(n, n, dtype=torch.float64, device=cuda, generator=g)
+    A.diagonal().add_(2.0 * n)                                  # dominant: no growth, |L| |U| below 2 |A|
+    At, piv = A.t().contiguous(), torch.zeros(n, dtype=torch.int32, device=cuda)
+    lnb.dgetrf_dev(At, n, n, piv)
+    B = torch.randn(nrhs, n, dtype=torch.float64, device=cuda, generator=g)
+    Bt = B.clone()
+    torch.cuda.synchronize()
+    assert lib.lnb_selftest_wait_timeout(5000) == -5
+    lnb.dgetrs_dev(At, piv, Bt, n, nrhs)
+    scale = 2 * float(A.abs().sum(1).max() * Bt.abs().max()) + float(B.abs().max())
+    assert float((Bt @ A.T - B).abs().max()) <= 12 * (n + 64) * U * scale
+
+
 # ---------------------------------------------------------------- products
 @pytest.mark.parametrize("ta,tb", [(a, b) for a in "NT" for b in "NT"])
 @pytest.mark.parametrize("m,n,k,pad,off", [(1, 1, 1, 0, 0), (64, 64, 16, 0, 0), (65, 63, 17, 1, 1), (130, 70, 15, 0, 1),
