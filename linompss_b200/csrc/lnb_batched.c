@@ -4,8 +4,11 @@
  * One call = two launches on the caller's stream: a device-side counting sort
  * of the systems by size (largest first) and the persistent solver
  * (k_batched.cu).  Nothing synchronizes the host, so the call can be
- * captured in a CUDA graph once the workspace exists (any earlier call, or
- * lnb_batched_autotune, creates it).
+ * captured in a CUDA graph once the workspace exists (any earlier call of the
+ * mode, or lnb_batched_autotune, creates it: its size does not depend on the
+ * launch shape, and the order's 4 bytes per system fit the workspace's slack up
+ * to millions of systems).  A graph is valid until a call of another kind makes
+ * the workspace grow, or lnb_release_workspace.
  *
  * Autotuning: lnb_batched_autotune times the candidate launch shapes on the
  * caller's own batch and keeps the fastest for the rest of the process:
@@ -65,7 +68,9 @@ static int batched_run(int count, const int *n, const int *nrhs, const int64_t *
     const int fp64 = mode == LNB_FACTOR_FP64;
     const bcfg cf = shape ? *shape : shape_of(c, mode, count);
     const int grid = c->sms * cf.per_sm;
-    const size_t sb = lnb_batched_scratch_bytes(grid, fp64);
+    /* for the most systems per SM that any shape of the mode runs: a small batch's
+     * workspace then serves a larger one, also one that is being captured */
+    const size_t sb = lnb_batched_scratch_bytes(c->sms * (fp64 ? 1 : 2), fp64);
     void *ws = lnb_ws(c, lnb_align256(sb) + lnb_align256((size_t)count * 4) + 512);
     if (!ws) return LNB_ENOMEM;
     lnb_arena ar = {(char *)ws, 0, c->ws_size};

@@ -175,3 +175,43 @@ def test_batched_not_spd_at_every_panel_position(lnb, cuda, mode):
     got = info.cpu().numpy()
     assert list(got[:len(bad_cols)]) == [c + 1 for c in bad_cols]
     assert (got[len(bad_cols):] == 0).all()
+
+
+@pytest.mark.parametrize("captured,eager", [(700, 40), (40, 700)])
+def test_batched_capture_without_autotuning(captured, eager):
+    """The launch shape follows the count; the workspace does not.  A call of one shape is captured after a call of
+    the other has made the workspace, and the replay, after one more call of the other shape, solves its batch.  In a
+    process of its own: untuned, and no other entry point has made the workspace larger."""
+    import os
+    import subprocess
+    import sys
+    code = f"""
+import sys
+sys.path.insert(0, "tests")
+import torch
+import linompss_b200 as lnb
+from test_gpu_batched import check, make_batch, to_device
+dev = torch.device("cuda:0")
+s = torch.cuda.Stream()
+b = [make_batch(c, seed=c, nmin=8, nmax=96) for c in ({captured}, {eager})]
+d = [to_device(*x, dev) for x in b]
+X = [torch.zeros_like(x[5]) for x in d]
+run = lambda k: lnb.batched_posv_dev(*d[k][:6], X[k], lnb.FACTOR_FP32, 10, stream=s)
+g = torch.cuda.CUDAGraph()
+with torch.cuda.stream(s):
+    run(1)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=s):
+        run(0)
+    X[1].zero_()
+    run(1)
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+for k in (0, 1):
+    assert check(*b[k], X[k].cpu().numpy(), d[k][6]) <= 10.0, k
+print("both solved")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "both solved" in r.stdout, r.stdout + r.stderr
