@@ -14,6 +14,7 @@
  * calls of several host threads.  Small copies, and copies of memory that is
  * pinned, managed or on a device, take the driver's path as before.
  */
+#include <cuda.h>
 #include <pthread.h>
 #include <stdatomic.h>
 #include <string.h>
@@ -35,6 +36,8 @@ typedef struct {
     cudaStream_t s;
     atomic_long next;           /* the next column, counted through all rectangles in chunks */
     atomic_int err;
+    CUcontext ctx;              /* the caller's: the streams and events belong to it */
+    CUresult (*set_current)(CUcontext);
 } stage_job;
 
 typedef struct {
@@ -85,7 +88,9 @@ static void *stage_run(void *arg)
     lnb_ctx *c = j->c;
     const lnb_rect *r[2] = {NULL, NULL};
     size_t col[2] = {0, 0}, ncol[2] = {0, 0};
-    int e = (int)cudaSetDevice(c->device);
+    /* The started threads join the caller's context, which need not be the device's primary
+     * one (cudaSetDevice would make that current); the caller's own thread has it. */
+    int e = me->w && j->set_current(j->ctx) != CUDA_SUCCESS ? (int)cudaErrorInvalidResourceHandle : 0;
     for (int k = 0; !e; k ^= 1) {
         const int slot = 2 * me->w + k;
         char *buf = (char *)c->stage + (size_t)slot * STAGE_CHUNK;
@@ -114,6 +119,20 @@ static void *stage_run(void *arg)
         }
     if (e) atomic_store(&j->err, e);
     return NULL;
+}
+
+/* the driver's functions for the current context of a thread; 0 if they cannot be had */
+static int context_calls(CUcontext *now, CUresult (**set_current)(CUcontext))
+{
+    void *get = NULL, *set = NULL;
+    enum cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &get, cudaEnableDefault, &q) != cudaSuccess || !get ||
+        cudaGetDriverEntryPoint("cuCtxSetCurrent", &set, cudaEnableDefault, &q) != cudaSuccess || !set) {
+        cudaGetLastError();
+        return 0;
+    }
+    *set_current = (CUresult (*)(CUcontext))set;
+    return ((CUresult (*)(CUcontext *))get)(now) == CUDA_SUCCESS;
 }
 
 static int is_pageable(const void *p)
@@ -158,6 +177,7 @@ int lnb_copy_rects(lnb_ctx *c, const lnb_rect *r, int nr, size_t dpitch, size_t 
             stage_job j = {.c = c, .r = r, .nr = nr, .to_device = to_device, .dpitch = dpitch, .hpitch = hpitch, .s = s};
             stage_worker w[STAGE_THREADS];
             int nt = cpus - 1 < STAGE_THREADS ? (int)cpus - 1 : STAGE_THREADS, started = 1;
+            if (!context_calls(&j.ctx, &j.set_current)) nt = 1;
             atomic_init(&j.next, 0);
             atomic_init(&j.err, 0);
             for (int i = 0; i < nt; ++i) {

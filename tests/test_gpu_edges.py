@@ -522,3 +522,33 @@ def test_host_calls_from_several_threads(lnb):
     assert len(out) == 3
     for rc, berr, m in out:
         assert rc == 0 and berr <= 12 * (m + 64) * U
+
+
+def test_host_copies_keep_the_callers_context(lnb):
+    """A program with a CUDA context of its own (not the device's primary one): large pageable copies run in it, and it
+    is current again, or rather still, after the call"""
+    import os
+    import subprocess
+    import sys
+    code = """
+import ctypes as C, sys
+import numpy as np
+cu = C.CDLL("libcuda.so.1")
+ctx, dev, now = C.c_void_p(), C.c_int(), C.c_void_p()
+assert cu.cuInit(0) == 0 and cu.cuDeviceGet(C.byref(dev), 0) == 0
+assert cu.cuCtxCreate_v2(C.byref(ctx), 0, dev) == 0
+import linompss_b200 as lnb
+m = 1100
+T = np.asfortranarray(np.tril(np.random.default_rng(0).standard_normal((m, m))) / 30 + 4 * np.eye(m))
+B0 = np.asfortranarray(np.random.default_rng(1).standard_normal((m, m)))
+for _ in range(2):
+    B = B0.copy(order="F")
+    rc = lnb.ompss_dtrsm("L", "L", "N", "N", m, m, 64, 1.0, T, m, B, m)
+    assert rc == 0, (rc, lnb.last_error())
+    assert cu.cuCtxGetCurrent(C.byref(now)) == 0 and now.value == ctx.value, "another context is current"
+    assert np.abs(T @ B - B0).max() <= 1e-11
+print("same context")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same context" in r.stdout, r.stdout + r.stderr
