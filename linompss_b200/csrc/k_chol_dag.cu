@@ -817,9 +817,12 @@ __global__ void __launch_bounds__(NTHR, CPS) k_chol_dag_f64(Args a)
             if (warp < NT / 32) warm_factor(a, j, sm, sh);
             __syncthreads();                         // before the producer's copies
         }
-        if (warp == NT / 32 ? !produce(a, kind, i, j, vec, sm, sh, n) : !multiply(a, kind, i, j, sm, sh, n))
+        if (warp == NT / 32 ? !produce(a, kind, i, j, vec, sm, sh, n) : !multiply(a, kind, i, j, sm, sh, n)) {
+            if (threadIdx.x == 0) give_up(a, 34, j * a.nt + i);   // stands unless the producer's own wait ran out
             sh.abort = 1;
+        }
     }
+    cp_async_wait<0>();                              // what the producer issued for a task that gave up
 }
 
 }  // namespace dag

@@ -104,6 +104,10 @@ LNB_DEV int wait_prog(const int *f, int target, const Args &a)
         if (it > 8) __nanosleep(40);
     }
 }
+LNB_DEV void give_up(const Args &a, int site, int item)
+{
+    if (atomicCAS(&a.st->timeout, 0, site) == 0) a.st->timeout_item = item;
+}
 LNB_DEV void arrive_copied(uint64_t *bar)
 {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -240,7 +244,7 @@ LNB_DEV bool produce(const Args &a, int v, int s, double *sm, Shared &sh, int &q
     }
     if (!ok) {
         if (lane == 0) {
-            if (atomicCAS(&a.st->timeout, 0, 51) == 0) a.st->timeout_item = v * a.ns + s;
+            give_up(a, 51, v * a.ns + s);
             sh.abort = 1;
         }
         cp_async_wait<0>();
@@ -395,9 +399,12 @@ __global__ void __launch_bounds__(NTHR, 2) k_trsm_tiles(Args a)
         const int tk = sh.task;
         if (tk >= a.ntasks) break;
         const int v = tk / a.ns, s = tk - v * a.ns;
-        if (warp == NT / 32 ? !produce<NW, TR>(a, v, s, sm, sh, q) : !multiply<NW, TR>(a, v, s, sm, sh, q, nd))
+        if (warp == NT / 32 ? !produce<NW, TR>(a, v, s, sm, sh, q) : !multiply<NW, TR>(a, v, s, sm, sh, q, nd)) {
+            if (threadIdx.x == 0) give_up(a, 52, v * a.ns + s);   // stands unless the producer's own wait ran out
             sh.abort = 1;
+        }
     }
+    cp_async_wait<0>();                              // what the producer issued for a task that gave up
 }
 
 template <int NW>
