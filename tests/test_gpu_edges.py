@@ -373,6 +373,51 @@ def test_syrk_edges(lnb, cuda, uplo, trans, n, k, pad, off):
     assert (err <= 2 * (k + 4) * U * (0.5 * np.abs(a) @ np.abs(a).T + 2 * np.abs(Cm))).all()
 
 
+# the larger launch forms: K split over clusters of 8, 4 and 2 (few tiles, deep K), three CTAs per SM with the per-thread
+# copy places (297 to 444 CTAs, alone and with K split; more than 592), the four-stage form between; odd leading
+# dimensions, 8-byte bases and ragged K in each
+@pytest.mark.parametrize("ta,tb", [(a, b) for a in "NT" for b in "NT"])
+@pytest.mark.parametrize("m,n,k,pad,off", [(130, 70, 1040, 1, 1), (130, 70, 5035, 0, 0), (130, 130, 1001, 1, 0),
+                                           (900, 800, 301, 1, 1), (900, 800, 300, 0, 0), (1281, 1025, 37, 1, 1),
+                                           (1281, 1025, 50, 0, 0), (1500, 1300, 51, 1, 0), (1601, 1601, 131, 1, 1),
+                                           (1602, 1601, 130, 0, 0), (1601, 1602, 15, 3, 0)])
+def test_gemm_launch_forms(lnb, cuda, ta, tb, m, n, k, pad, off):
+    import torch
+    rng = np.random.default_rng(m + n + k)
+    A = rng.standard_normal((m, k) if ta == "N" else (k, m))
+    B = rng.standard_normal((k, n) if tb == "N" else (n, k))
+    Cm = rng.standard_normal((m, n))
+    At, _ = dev(cuda, A, A.shape[0] + pad, off)
+    Bt, _ = dev(cuda, B, B.shape[0] + pad, off)
+    Ct, _ = dev(cuda, Cm, m + pad, off)
+    lnb.dgemm_dev(ta, tb, m, n, k, -1.25, At, Bt, 0.75, Ct)
+    a, b, c = (torch.tensor(np.ascontiguousarray(x), device=cuda) for x in (A, B, Cm))
+    a, b = (a if ta == "N" else a.T), (b if tb == "N" else b.T)
+    bound = 2 * (k + 4) * U * (1.25 * a.abs() @ b.abs() + 0.75 * c.abs())
+    assert bool((Ct[:, m:] == 7.25).all())
+    assert bool(((Ct[:, :m].T - (-1.25 * (a @ b) + 0.75 * c)).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("uplo,trans", [(a, b) for a in "LU" for b in "NT"])
+@pytest.mark.parametrize("n,k,pad,off", [(220, 5035, 1, 1), (220, 1008, 0, 0), (900, 401, 1, 0), (1200, 301, 1, 1),
+                                         (1801, 37, 1, 1), (1800, 50, 0, 0), (2000, 51, 1, 0), (2301, 37, 1, 1),
+                                         (2302, 130, 0, 0)])
+def test_syrk_launch_forms(lnb, cuda, uplo, trans, n, k, pad, off):
+    import torch
+    rng = np.random.default_rng(n + k)
+    A = rng.standard_normal((n, k) if trans == "N" else (k, n))
+    Cm = rng.standard_normal((n, n))
+    At, _ = dev(cuda, A, A.shape[0] + pad, off)
+    Ct, _ = dev(cuda, Cm, n + pad, off)
+    lnb.dsyrk_dev(uplo, trans, n, k, 0.5, At, -2.0, Ct)
+    a, c = (torch.tensor(np.ascontiguousarray(x), device=cuda) for x in (A if trans == "N" else A.T, Cm))
+    half = torch.tril if uplo == "L" else torch.triu
+    got = Ct[:, :n].T
+    assert bool((Ct[:, n:] == 7.25).all()) and torch.equal(got - half(got), c - half(c))
+    bound = 2 * (k + 4) * U * (0.5 * a.abs() @ a.abs().T + 2 * c.abs())
+    assert bool((half(got - (0.5 * a @ a.T - 2.0 * c)).abs() <= bound).all())
+
+
 # one term per element, so the sum is exact up to its one rounding, and the last step is visible: alpha P is not
 # rounded before beta C joins.  m, n, k reach one CTA's form, K split over a cluster, and three CTAs per SM
 @pytest.mark.parametrize("m,n,k", [(65, 63, 1), (200, 100, 2100), (1500, 1400, 3)])
@@ -440,6 +485,25 @@ def test_dcg_edges(lnb, n, steps):
     rco, xo, _ = O.cg(A, rhs, 32, 1e-14, steps)
     assert rc == rco
     np.testing.assert_allclose(x, xo, rtol=0, atol=2 * (n + 8) * U * 4.0 ** max(steps, 1) * max(np.abs(xo).max(), 1e-300))
+
+
+@pytest.mark.parametrize("n", [12288, 12289])
+def test_dcg_largest_one_launch(lnb, n):
+    """the largest order of the one-launch form, and the next; A = 3 I + a rank-one term, condition number below 4"""
+    rng = np.random.default_rng(n)
+    v = rng.uniform(-1, 1, n)
+    A = np.empty((n, n), order="F")
+    np.multiply.outer(v, v * (3.0 / n), out=A.T)               # symmetric in exact arithmetic; the upper triangle copied
+    for r in range(0, n, 2048):
+        A[r:, r:r + 2048] = A[r:r + 2048, r:].T.copy()
+        B = A[r:r + 2048, r:r + 2048]
+        B[:] = np.triu(B) + np.triu(B, 1).T
+    A[np.arange(n), np.arange(n)] += 3
+    rhs, x, steps = rng.standard_normal(n), np.zeros(n), 3
+    rc = lnb.ompss_dcg(n, 512, A, n, rhs.copy(), x, 1e-14, steps)
+    rco, xo, _ = O.cg(A, rhs, 512, 1e-14, steps)
+    assert rc == rco
+    np.testing.assert_allclose(x, xo, rtol=0, atol=2 * (n + 8) * U * 4.0 ** steps * np.abs(xo).max())
 
 
 # ---------------------------------------------------------------- batched solves: both launch shapes
