@@ -8,7 +8,7 @@
 //           permutation of the at most 2 nb rows they touch.
 //   apply : the panel's swaps on other columns, and right of the panel the
 //           unit-lower solve of its rows and the update of the rows below, on
-//           DMMA, in one launch.
+//           DMMA, in one launch (above 24576 rows the update is a product of its own).
 //   laswp : row swaps given as pivots, on any columns.
 #include <cooperative_groups.h>
 #include <stdlib.h>
@@ -600,11 +600,20 @@ extern "C" int lnb_k_lu_apply_f64(double *A, int64_t lda, int64_t m, int64_t c0,
     if (nb > MAXNB) return (int)cudaErrorInvalidValue;
     const unsigned grid = (unsigned)(nl + nr);
     if (a1 < a0) a1 = a0;
-    if (nb > 8) k_lu_apply<16><<<grid, AT, 0, (cudaStream_t)s>>>(A, lda, m, c0, nb, (const Perm *)perm, a0, a1, b0, b1);
-    else if (nb > 4) k_lu_apply<8><<<grid, AT, 0, (cudaStream_t)s>>>(A, lda, m, c0, nb, (const Perm *)perm, a0, a1, b0, b1);
-    else k_lu_apply<4><<<grid, AT, 0, (cudaStream_t)s>>>(A, lda, m, c0, nb, (const Perm *)perm, a0, a1, b0, b1);
+    /* Panels of 4 columns (more than 24576 rows): a CTA per 8 columns would run through all the rows for
+       a rank-4 step, and inside a 256-column block there are at most 32 such CTAs.  The product's tiles fill
+       the chip: 32768 x 256, mean per panel, 119 us in one launch, 7 + 74 as two (panels of 8 columns, 24576 x
+       256: 95 in one launch against about 2 x 65). */
+    const bool split = lnb_lu_panel_width(m - c0) <= 4 && b1 > b0 && m > c0 + nb;
+    const int64_t mu = split ? c0 + nb : m;
+    if (nb > 8) k_lu_apply<16><<<grid, AT, 0, (cudaStream_t)s>>>(A, lda, mu, c0, nb, (const Perm *)perm, a0, a1, b0, b1);
+    else if (nb > 4) k_lu_apply<8><<<grid, AT, 0, (cudaStream_t)s>>>(A, lda, mu, c0, nb, (const Perm *)perm, a0, a1, b0, b1);
+    else k_lu_apply<4><<<grid, AT, 0, (cudaStream_t)s>>>(A, lda, mu, c0, nb, (const Perm *)perm, a0, a1, b0, b1);
     lnb_prof_count(1);
-    return (int)cudaGetLastError();
+    const int e = (int)cudaGetLastError();
+    if (e || !split) return e;
+    return lnb_k_gemm_tri_f64('N', 'N', m - c0 - nb, b1 - b0, nb, -1.0, A + (c0 + nb) + c0 * lda, lda, A + c0 + b0 * lda,
+                              lda, 1.0, A + (c0 + nb) + b0 * lda, lda, 0, s);
 }
 
 extern "C" int lnb_k_laswp_f64(double *A, int64_t lda, int64_t k0, int64_t k1, const int *piv, int64_t a0,

@@ -38,6 +38,7 @@
     } while (0)
 
 #define LU_BO 256
+#define LU_ONE_CHUNK 32
 /* up to this many elements (64 MB, half the L2 cache) every panel updates all
  * the columns right of it: the rank-16 passes over the matrix stay in L2 */
 #define LU_ONE_LEVEL (8LL << 20)
@@ -125,7 +126,8 @@ static int getrs_run(lnb_ctx *c, int64_t n, int64_t nrhs, const double *dLU, int
     int *src = lnb_arena_take(&a2, (size_t)n * 4);
     double *T = lnb_arena_take(&a2, (size_t)n * getrs_cols(n, nrhs) * 8);
     if (!src || !T) return lnb_set_error(LNB_ENOMEM, "getrs workspace");
-    if (n <= lnb_rows_permute_max())
+    /* up to 32 rows are one chunk of swaps, in one launch instead of three */
+    if (n > LU_ONE_CHUNK && n <= lnb_rows_permute_max())
         CK(lnb_k_rows_permute_f64(dB, ldb, n, nrhs, n, dpiv, src, T, getrs_cols(n, nrhs), s), "rhs swaps");
     else
         CK(lnb_k_laswp_f64(dB, ldb, 0, n, dpiv, 0, nrhs, 0, 0, s), "rhs swaps");
