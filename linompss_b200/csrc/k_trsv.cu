@@ -100,20 +100,23 @@ __global__ void __launch_bounds__(TI_NT) k_trtri_blocks(const TT *T, int64_t ldt
             if (r >= c) X[(b0 + r) * TI_LD + b0 + c] = x[r];
     }
     __syncthreads();
-    // 16 -> 32: C A^-1 into the unused upper block of L, then -D^-1 (C A^-1)
-    {
+    // (a step whose lower rows are all padding would fill in zeros: skipped)
+    if (qn > 16) {
+        // 16 -> 32: C A^-1 into the unused upper block of L, then -D^-1 (C A^-1)
         const int b0 = tid < TI_NT / 2 ? 0 : 32, p = tid % (TI_NT / 2);
         double *Lb = L + b0 * TI_LD + b0, *Xb = X + b0 * TI_LD + b0;
         ti_product(Lb + 16, Lb + 16 * TI_LD, Xb, 16, 1.0, p, TI_NT / 2);
         __syncthreads();
         ti_product(Xb + 16 * TI_LD, Xb + 16 * TI_LD + 16, Lb + 16, 16, -1.0, p, TI_NT / 2);
+        __syncthreads();
     }
-    __syncthreads();
-    // 32 -> 64
-    ti_product(L + 32, L + 32 * TI_LD, X, 32, 1.0, tid, TI_NT);
-    __syncthreads();
-    ti_product(X + 32 * TI_LD, X + 32 * TI_LD + 32, L + 32, 32, -1.0, tid, TI_NT);
-    __syncthreads();
+    if (qn > 32) {
+        // 32 -> 64
+        ti_product(L + 32, L + 32 * TI_LD, X, 32, 1.0, tid, TI_NT);
+        __syncthreads();
+        ti_product(X + 32 * TI_LD, X + 32 * TI_LD + 32, L + 32, 32, -1.0, tid, TI_NT);
+        __syncthreads();
+    }
     TT *D = dinv + (int64_t)q * TH * TH;           // column-major
     for (int idx = tid; idx < TH * TH; idx += TI_NT) {
         const int c = idx / TH, r = idx % TH;
