@@ -351,7 +351,9 @@ LNB_EXPORT int lnb_batched_posv_dev(int count, const int *n_dev, const int *nrhs
  * SM (1 / 2) and processing order (largest first / largest and smallest
  * interleaved), and keeps the fastest for later lnb_batched_posv_dev calls of
  * the same mode.  Returns the chosen CTA size; lnb_batched_config reports the
- * whole shape.  Each system's A_s is n x n FP64 with both triangles stored. */
+ * whole shape.  (Before autotuning, FP32 batches of at most four systems per SM
+ * run with 512 threads and one system per SM; lnb_batched_config reports the
+ * shape of larger ones.)  Each system's A_s is n x n FP64 with both triangles stored. */
 LNB_EXPORT int lnb_batched_autotune(int count, const int *n_dev, const int *nrhs_dev,
                                     const int64_t *a_off_dev, const int64_t *b_off_dev,
                                     const double *dA, const double *dB, double *dX,

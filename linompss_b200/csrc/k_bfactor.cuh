@@ -293,8 +293,10 @@ LNB_DEV void bblock(const TF *sD, double *z, int k0, int kn, int nr)
 // row with the block's 32 entries of that row in flight; backward, a warp sums a
 // few columns below the block, all its lanes' partial sums folded in one pass.
 // (Forward as a sum per block, reduced over the warps, had 4 loads in flight and
-// two more barriers per block: 10,000 systems of n <= 512 took 30.6 ms, now 29.8.
-// Both directions are chains of block steps, 4 K cycles each.)
+// two more barriers per block: 10,000 systems of n <= 512 took 30.6 ms, then 29.8.
+// Both directions are chains of block steps, 4 K cycles each.)  The last block has no
+// rows below it to fetch, and its inverse stays in place for the backward solve: one
+// system of n <= 32 went from 49 us to 45.
 template <typename TF, int NT>
 __device__ void bsolve(const TF *F, int ldF, const TF *Dv, int n, int nr, double *z, TF *sD,
                        const int *env = nullptr)
@@ -319,7 +321,7 @@ __device__ void bsolve(const TF *F, int ldF, const TF *Dv, int n, int nr, double
 #pragma unroll
             for (int c = 0; c < BP; ++c) f[c] = in && c < kn ? __ldcg(F + r + (int64_t)(k0 + c) * ldF) : TF(0);
         };
-        fetch();
+        if (k1 < re) fetch();
         bblock<TF, false>(sD + (kb & 1) * DB, z, k0, kn, nr);
         __syncthreads();
         while (r < re) {
@@ -344,11 +346,9 @@ __device__ void bsolve(const TF *F, int ldF, const TF *Dv, int n, int nr, double
             if (r < re) fetch();
         }
     }
-    // backward
-    __syncthreads();
+    // backward; the last block's inverse is still in its place
     constexpr int CPW = BP / NW, V = CPW * BMAXR;          // columns of a block per warp
     static_assert(V == 32 || V == 16, "8 or 16 warps");
-    bstage_inv<TF, NT>(sD + ((nblk - 1) & 1) * DB, Dv + (int64_t)(nblk - 1) * BP * BP);
     for (int kb = nblk - 1; kb >= 0; --kb) {
         const int k0 = kb * BP, kn = min(BP, n - k0), r0 = k0 + kn;
         const int re = env ? min(n, env[BMAXN / BP + kb] + 1) : n;    // rows from re on are zero here

@@ -41,12 +41,20 @@ typedef struct { int nt, per_sm, interleave; } bcfg;
 static bcfg g_cfg[2] = {{256, 2, 0}, {256, 1, 0}};   /* [fp32 mode, fp64 mode] */
 static int g_tuned[2];                               /* g_cfg is the autotuner's */
 
-/* The launch shape of an untuned batch.  FP32: two systems of 256 threads per SM
- * hide each other's latency once every SM has several; a smaller batch wants each
- * system done sooner, with 512 threads.  Measured, ms at (256, 1) / (256, 2) /
- * (512, 1), n <= 512: 10000 systems 46.0 / 30.6 / 35.0, 2000 9.20 / 6.24 / 7.04, 600
- * 2.97 / 2.49 / 2.25, 300 1.77 / 2.12 / 1.31, 60 1.36 / 1.45 / 1.10; 9000 of n <= 100
- * 5.11 / 2.90 / 5.30. */
+/* The launch shape of an untuned batch, which must not depend on the orders (they are on
+ * the device).  FP32: two systems of 256 threads per SM hide each other's latency once
+ * every SM has several; a smaller batch wants each system done sooner, with 512
+ * threads.  Measured, us at (256, 1) / (256, 2) / (512, 1), one right-hand side:
+ *   orders     148 systems         296                 593                 1500
+ *   8-32         49 /   53 /   49    70 /   55 /   70    127 /  82 /  129    293 /  176 /  299
+ *   16-100      145 /  154 /  139   174 /  154 /  170    330 / 195 /  322    758 /  437 /  735
+ *   16-256      409 /  481 /  369   422 /  510 /  377    803 / 545 /  754   1942 / 1210 / 1786
+ *   16-512     1485 / 1907 / 1167  1602 / 2149 / 1241   2471 / 2383 / 2009  6158 / 4330 / 4974
+ *   400-512    1649 / 2245 / 1272  2821 / 2464 / 2145   6146 / 4612 / 4753 14259 /10518 /10928
+ * The line at four systems per SM: below it (256, 2) loses up to 1.5 times against 512
+ * threads where the orders reach 512; from it on it loses 1.2 there and wins 1.4 to 1.7 on
+ * small orders.  (512, 1) is never behind (256, 1) by more than their spread.  The
+ * autotuner, which sees the batch, replaces the rule. */
 static bcfg shape_of(const lnb_ctx *c, int mode, int count)
 {
     const int k = mode == LNB_FACTOR_FP64;
@@ -92,6 +100,7 @@ int lnb_batched_posv_dev(int count, const int *n_dev, const int *nrhs_dev, const
                        iters_dev, (cudaStream_t)stream, NULL);
 }
 
+/* the shape in use, for an untuned FP32 mode that of batches above the line */
 int lnb_batched_config(int mode, int *cta_threads, int *ctas_per_sm, int *interleave)
 {
     const bcfg cf = g_cfg[mode == LNB_FACTOR_FP64];
