@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(128) k_trsm_rlt_f64(const double *__restrict__
 // cp.async along a column: op(A) = A and op(B) = B^T are stored k-major
 // (S[k][m], row stride 68), op(A) = A^T and op(B) = B m-major (S[m][k], row
 // stride 20).  Both strides spread a half-warp's fragment reads over all 32
-// banks.  beta == 0 does not read C (BLAS semantics); alpha times the sum is not
-// rounded before beta C joins it (fma).
+// banks.  beta == 0 does not read C (BLAS semantics); beta C is not rounded before it
+// joins alpha times the sum (fma).
 // Bound by the DMMA rate once three CTAs share every SM: there a thread's places in a
 // chunk, its pointers and its rows' predicates are set once (Loader) and a chunk costs
 // four copies per operand; with them computed per copy (load_op) only two CTAs fit
@@ -543,10 +543,10 @@ __global__ void __launch_bounds__(THREADS, DEEP ? 2 : 3) k_gemm_dmma(int64_t M, 
             double *cp = C + r0 + c0 * ldc;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                cv[q] = beta != 0.0 && keep(q) ? beta * cp[(q >> 1) * 8 + (q & 1) * ldc] : 0.0;
+                cv[q] = beta != 0.0 && keep(q) ? cp[(q >> 1) * 8 + (q & 1) * ldc] : 0.0;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                if (keep(q)) cp[(q >> 1) * 8 + (q & 1) * ldc] = fma(alpha, v[q], cv[q]);
+                if (keep(q)) cp[(q >> 1) * 8 + (q & 1) * ldc] = fma(beta, cv[q], __dmul_rn(alpha, v[q]));
         }
         cl.sync();                                 // no CTA leaves while its part may be read
     } else {
@@ -565,13 +565,14 @@ __global__ void __launch_bounds__(THREADS, DEEP ? 2 : 3) k_gemm_dmma(int64_t M, 
             for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    cv[ni][q] = beta != 0.0 && keep(ni, q) ? beta * cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] : 0.0;
+                    cv[ni][q] = beta != 0.0 && keep(ni, q) ? cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] : 0.0;
 #pragma unroll
             for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
                     if (keep(ni, q))
-                        cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] = fma(alpha, acc[mi][ni][q], cv[ni][q]);
+                        cp[(q >> 1) * 8 + (ni * 8 + (q & 1)) * ldc] =
+                            fma(beta, cv[ni][q], __dmul_rn(alpha, acc[mi][ni][q]));
         }
     }
 }

@@ -418,8 +418,8 @@ def test_syrk_launch_forms(lnb, cuda, uplo, trans, n, k, pad, off):
     assert bool((half(got - (0.5 * a @ a.T - 2.0 * c)).abs() <= bound).all())
 
 
-# one term per element, so the sum is exact up to its one rounding, and the last step is visible: alpha P is not
-# rounded before beta C joins.  m, n, k reach one CTA's form, K split over a cluster, and three CTAs per SM
+# one term per element, so the sum is exact up to its one rounding, and the last step is visible: beta C is not
+# rounded before it joins alpha P.  m, n, k reach one CTA's form, K split over a cluster, and three CTAs per SM
 @pytest.mark.parametrize("m,n,k", [(65, 63, 1), (200, 100, 2100), (1500, 1400, 3)])
 @pytest.mark.parametrize("beta", [0.0, 0.7])
 def test_gemm_epilogue_is_fused(lnb, cuda, m, n, k, beta):
@@ -435,7 +435,7 @@ def test_gemm_epilogue_is_fused(lnb, cuda, m, n, k, beta):
     got = Ct.cpu().numpy().T
     for r, c in zip(rng.integers(0, m, 2000), rng.integers(0, n, 2000)):
         p = A[r, k // 2] * B[k // 2, c]
-        assert got[r, c] == float(Fraction(alpha) * Fraction(p) + Fraction(beta * Cm[r, c])), (r, c)
+        assert got[r, c] == float(Fraction(alpha * p) + Fraction(beta) * Fraction(Cm[r, c])), (r, c)
 
 
 def test_gemm_from_two_threads(lnb, cuda):
