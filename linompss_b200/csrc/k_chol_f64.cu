@@ -576,20 +576,21 @@ __global__ void __launch_bounds__(THREADS, DEEP ? 2 : 3) k_gemm_dmma(int64_t M, 
         }
     }
 }
+constexpr int SMS = 148;                           // a B200's; the lines below were measured there
 // Parts K is split into: as many (8, 4 or 2) as keep all CTAs resident, three on each of
-// the 148 SMs, with 128 or more of K each.  SYRK in one part / split, start to end:
+// the SMs, with 128 or more of K each.  SYRK in one part / split, start to end:
 // n = 220, k = 5035 (10 tiles) 336 us / 46 in eight; n = k = 500 (36) 45 / 19 in four;
 // n = k = 1000 (136) 91 / 52 in two.
 inline int splits(int64_t tiles, int64_t K)
 {
     const int64_t kt = (K + BK - 1) / BK;
     for (int S = 8; S > 1; S /= 2)
-        if (tiles * S <= 3 * 148 && kt / S >= 8) return S;
+        if (tiles * S <= 3 * SMS && kt / S >= 8) return S;
     return 1;
 }
 // Four stages and two CTAs per SM where three CTAs per SM would not fill the chip, or would
 // leave a nearly empty second wave (n = 1900, k = 3000, 465 tiles: 482 us, with three 596).
-inline bool deep(int64_t ctas) { return ctas <= 2 * 148 || (ctas > 3 * 148 && ctas <= 4 * 148); }
+inline bool deep(int64_t ctas) { return ctas <= 2 * SMS || (ctas > 3 * SMS && ctas <= 4 * SMS); }
 }  // namespace gm
 
 }  // namespace lnb
@@ -674,7 +675,7 @@ static int launch_gemm_as(dim3 grid, int64_t m, int64_t n, int64_t k, double alp
        SM do not fill every SM (144 CTAs by fours took two waves), so only up to 96 CTAs. */
     const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
     constexpr int ONE = 116 * 1024, TWO = SMEM > 80 * 1024 ? SMEM : 80 * 1024;
-    const int smem = !DEEP ? SMEM : ctas <= (SPLIT ? 96 : 148) ? ONE : TWO;
+    const int smem = !DEEP ? SMEM : ctas <= (SPLIT ? 96 : gm::SMS) ? ONE : TWO;
     /* always the most that any launch of this kernel asks for: calls of several host
        threads may stand between here and the launch */
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -77,8 +77,10 @@ int lnb_potrf_tile_f64(double *Akk, int64_t lda, int bs, int64_t row0, double *d
  * LNB_SCHED_AUTO picks by size: the device DAG up to LNB_DAG_AUTO_MAX_N.
  * The environment variable LNB_CHOL_SCHED ("dag" / "streams") overrides the
  * process-wide setting. */
-/* measured on B200 (b = 256 - 512): the DAG walk is ahead of the two-stream
- * schedule from n = 512 (0.37 vs 0.41 ms) to n = 16384 (53.1 vs 55.0 ms) */
+/* Measured on B200 (b = 256 - 512), ms, walk / two streams: n = 512 0.14 / 0.32, 4096 1.19 / 3.57,
+ * 16384 46.0 / 53.6, and above the line too, 24576 153 / 168, 32768 362 / 385.  The line is
+ * where the streams begin to pay for a pinned host matrix, whose finished panels they
+ * copy back beside the factorization; the device entry points have no such reason. */
 #define LNB_DAG_AUTO_MAX_N 16384
 static int g_sched = LNB_SCHED_AUTO;
 
