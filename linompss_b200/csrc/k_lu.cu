@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(PT, 1) k_lu_panel(double *A, int64_t lda, int6
             p = rank == 0 ? k : INT_MAX;
             if (lane == 0) atomicCAS(&st->timeout, 0, 41);
         }
+        double rp = 1.0 / __longlong_as_double((long long)key);      // 1 / |pivot|, beside the exchange of its row
         // 2. its row and the row k
         const bool own = p != INT_MAX && ((p - base) % PT) >> 5 == warp;
         if (own) {
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(PT, 1) k_lu_panel(double *A, int64_t lda, int6
             p = lane < ncl ? S.cidx[b][lane] : INT_MAX;
             key = lane < ncl ? S.ckey[b][lane] : 0ull;
             warp_best(key, p);
+            rp = 1.0 / __longlong_as_double((long long)key);
             prow = (const double *)S.crow[b][p / (PT * RPT)];
             krow = (const double *)S.ckrow[b];
         }
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(PT, 1) k_lu_panel(double *A, int64_t lda, int6
         // division per element 3.65.  A zero pivot divides nothing, as in dgetf2.
         const double apv = fabs(pv);
         const bool plain = apv >= 1e-280 && apv <= 1e280;
-        const double rp = 1.0 / pv;
+        rp = copysign(rp, pv);
         // 3. row p takes the old row k
         if (p >= base && p < base + PT * RPT && ((p - base) % PT) >> 5 == warp) {
 #pragma unroll
